@@ -33,8 +33,8 @@ typedef struct {
 
 /* y = act(conv3x3x3(x, w) + bias); act = ReLU when relu != 0.  wt is the
  * forward packing of nn_pack_weights.  Tensor cores with FP32 accumulation:
- * tcgen05.mma with a TMEM accumulator when the rows hold a multiple of 128
- * voxels (cout 16..64, 16-byte aligned views), mma.sync otherwise. */
+ * tcgen05.mma with TMEM accumulators for cout 16, 32, 48, 64, 96, 128 and 192
+ * on 16-byte aligned views (any grid), mma.sync otherwise. */
 int nn_conv3(const nn_act *x, const void *wt, const float *bias, const nn_act *y, int relu, void *stream);
 
 /* BBMG_CUDA if a tcgen05 convolution's completion wait ran out since the last

@@ -3,11 +3,12 @@
 // No counterpart in the reference (NGA2 starts each pressure solve from the
 // previous pressure).  The 3x3x3 convolutions (forward and data gradient) are
 // implicit GEMMs on the tensor cores: M = voxels, N = output channels, K = 27
-// taps x input channels, BF16 operands, FP32 accumulation.  Grids of whole
-// 128-voxel tiles run on tcgen05 (k_conv3_tcg: TMEM accumulator, cp.async
-// stage ring, one thread issuing the MMAs); other sizes on mma.sync m16n8k16
-// (k_conv3: a warp owns 16 consecutive voxels and all output channels, its A
-// fragments the tap-shifted input rows with periodic wrap, its B fragments the
+// taps x input channels, BF16 operands, FP32 accumulation.  They run on tcgen05
+// (k_conv3_zm: a column of voxel tiles per CTA, its accumulators in TMEM, input
+// planes staged once for all their taps); views that are not 16-byte aligned and
+// other output widths on mma.sync m16n8k16 (k_conv3: a warp owns 16 consecutive
+// voxels and all output channels, its A fragments the tap-shifted input rows
+// with periodic wrap, its B fragments the
 // packed weights).  The weight gradient, a contraction over voxels, runs on
 // mma.sync with ldmatrix.trans fragments (k_wgrad_mma); everything else is
 // elementwise.
@@ -118,28 +119,39 @@ __global__ void __launch_bounds__(128) k_conv3(Act x, const bf16 *__restrict__ w
 }
 
 // ---------------------------------------------------------------------------
-// The same convolution on the fifth-generation tensor cores (tcgen05): an
-// implicit GEMM with M = 128 consecutive voxels per CTA (one or more (h, w)
-// rows, or part of one), N = all output channels, K = 27 taps x cin.
-//   * K is walked in units of 16 channels (of one tap, or of one input row
-//     for three taps, below); a few units form a pipeline stage.  A stage holds the A tile (the 128 voxels' tap-shifted
-//     input channels, periodic wrap: thread m copies voxel m's two 16-byte
-//     chunks per step) and the B tile (the packed weights [tap][cout][cin] of
-//     those steps), both in the K-major no-swizzle canonical layout of the
-//     MMA: per 8-channel group, rows of 16 bytes one after another (A:
-//     [step][group][voxel][16 B], B: [step][group][cout][16 B]).
-//   * S stages (template parameter, 2 by default) form a ring filled with
-//     cp.async S-1 stages ahead; one
-//     thread issues the tcgen05.mma (M = 128, N = cout, K = 16, BF16 x BF16 ->
-//     FP32 in TMEM) of a stage and commits them to that stage's mbarrier; a
-//     stage is refilled once its mbarrier shows the MMAs reading it are done.
-//   * after the last stage the four warps read their 32 TMEM lanes (= 32
-//     voxels) with tcgen05.ld, add the bias, apply the ReLU, store BF16.
+// Convolution as implicit GEMM on the fifth-generation tensor cores (tcgen05).
+// A CTA owns a column of 8 (w) x 16 (h) voxels (M = 128) over up to DZ output
+// planes and all N = cout output channels; its FP32 accumulators, DZ x cout
+// columns, stay in TMEM.
+//   * K is walked in chunks of 16 input channels; a chunk marches over the
+//     DZ + 2 input planes.  A stage is one plane of one chunk: its 10 x 18
+//     voxels with the halo (periodic wrap), as [8-channel group][voxel][16 B],
+//     the K-major no-swizzle layout of the MMA with 160 bytes from one h row to
+//     the next.  Each of the nine (dy, dx) taps is then a descriptor shifted by
+//     whole 16-byte rows: every input element is read from global memory 1.4
+//     times per plane instead of once per tap.
+//   * Input plane p contributes to the output planes p-1, p, p+1 through the
+//     taps dz = +1, 0, -1.  Their accumulators are neighbouring TMEM columns and
+//     the chunk's weights are stored [dy, dx][group][dz][cout], so one MMA of
+//     N = 3 cout does all three: with 16 output channels an MMA's time is the
+//     reading of A (128 rows of 32 bytes at 128 B per cycle), whatever N.
+//     Where 3 cout > 256 the three go out one by one.
+//   * A planes sit in a ring of kZmA slots filled with cp.async kZmA - 1
+//     stages ahead; one thread issues a stage's MMAs and commits them to the
+//     slot's mbarrier, which gates its refill.  The weights of a chunk have NB
+//     buffers; with one, the next chunk's load waits for the MMAs before it.
+//   * The epilogue reads the four warps' 32 TMEM lanes, adds the bias, applies
+//     the ReLU and stores BF16.
+// Measured at 128^3 (the whole forward pass of the U-Net with its guess assembly):
+// 3.55 ms with one CTA per 128-voxel row tile that staged an input row for each
+// (dz, dy) and issued 27 MMAs of N = cout per tile, 1.71 ms with this kernel.
 // Every mbarrier wait is bounded: a wait that runs out raises *err (read by
-// nn_tc_error), and the CTA then drains its copies, frees its TMEM and
-// returns without writing.
+// nn_tc_error), and the CTA then drains its copies, frees its TMEM and returns
+// without writing.
 constexpr unsigned kTcSpinLimit = 1u << 22;
-constexpr int kTgS = 4;   // pipeline stages (the default of TgCfg; the launcher picks 2)
+constexpr int kZmA = 4;                     // A slots
+constexpr int kZmVox = 10 * 18;             // voxels of a halo plane
+constexpr int kZmPlane = kZmVox * 32;       // bytes of a stage's A
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -162,6 +174,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
+__device__ __forceinline__ void umma_bf16(unsigned tmem, uint64_t ad, uint64_t bd, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+        ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(1), "r"(0));
+}
+
 // bounded wait for the completion of phase `parity` of an mbarrier
 __device__ __forceinline__ bool mbar_wait(const uint64_t *mb, unsigned parity) {
     for (unsigned spins = 0; spins < kTcSpinLimit; spins++) {
@@ -176,158 +196,146 @@ __device__ __forceinline__ bool mbar_wait(const uint64_t *mb, unsigned parity) {
     return false;
 }
 
-// Two tilings.  ROW (rows of a multiple of 128 voxels): a tile is 128
-// consecutive voxels of one (n, d, h) row, and a K unit is one (dz, dy) input
-// row with its x-halo (130 voxels) for 16 channels: it is staged once and
-// serves the three dx taps through descriptors shifted by one 16-byte row
-// (three MMAs per unit).  Otherwise a tile is 128 consecutive voxels of the
-// grid (several rows when w < 128) and a K unit is one tap's 16 channels of
-// the 128 voxels (one MMA).
-template <int N, bool ROW, int S = kTgS>
-struct TgCfg {
-    static constexpr int kCols = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));  // TMEM columns
-    static constexpr int VOX = ROW ? 130 : 128;         // A rows staged per unit
-    static constexpr int TAPS = ROW ? 3 : 1;            // MMAs (taps) per unit
-    static constexpr int KU = ROW ? 2 : 4;              // units per stage
-    static constexpr int A_UNIT = 2 * VOX * 16;         // bytes: [group][voxel][16 B]
-    static constexpr int B_UNIT = TAPS * 2 * N * 16;    // bytes: [tap][group][cout][16 B]
-    static constexpr int A_BYTES = KU * A_UNIT;
-    static constexpr int B_BYTES = KU * B_UNIT;
-    static constexpr size_t SMEM = 128 + (size_t)S * (A_BYTES + B_BYTES);
+struct ZmGeo {
+    int tw, th, tz;  // tiles along w, h, d
+    int dz;          // output planes per tile
+    int cols;        // TMEM columns
+    int nb;          // weight buffers
 };
 
-template <int N, bool ROW, int S>
-__global__ void __launch_bounds__(128) k_conv3_tcg(Act x, const bf16 *__restrict__ wt, const float *__restrict__ bias,
-                                                    Act y, int relu, int *err) {
-    using Cfg = TgCfg<N, ROW, S>;
+__device__ __forceinline__ int wrapn(int i, int n) {
+    i %= n;
+    return i < 0 ? i + n : i;
+}
+
+template <int N>
+__global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict__ wt, const float *__restrict__ bias,
+                                                   Act y, int relu, ZmGeo geo, int *err) {
+    constexpr int kB = 27 * N * 32;  // bytes of a chunk's weights
     extern __shared__ __align__(128) unsigned char smtc[];
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(smtc);
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smtc + 16);  // S barriers
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smtc + 16);  // kZmA barriers
     unsigned char *A = smtc + 128;
-    unsigned char *B = A + (size_t)S * Cfg::A_BYTES;
+    unsigned char *B = A + (size_t)kZmA * kZmPlane;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int cin = x.c, kpt = cin >> 4;                 // 16-channel blocks
-    const int nu = (ROW ? 9 : 27) * kpt;                 // K units
-    const int nK = (nu + Cfg::KU - 1) / Cfg::KU;         // stages
-    int v0;              // first voxel of the tile
-    int vn[3], vd[3], vh[3], vw[3];
-    const int ag = tid & 1;  // A copies: chunk e = (voxel e/2, group e%2), e = tid + 128 r
-    if constexpr (ROW) {
-        const int tiles_per_row = x.w >> 7;
-        const int w0 = (blockIdx.x % tiles_per_row) << 7;
-        int rowid = blockIdx.x / tiles_per_row;
-        const int h = rowid % x.h;
-        rowid /= x.h;
-        const int d = rowid % x.d, n = rowid / x.d;
-        v0 = vox(x, n, d, h, w0);
-#pragma unroll
-        for (int u = 0; u < 3; u++) {  // halo voxel (tid>>1) + 64u of the row, x-wrapped
-            vn[u] = n; vd[u] = d; vh[u] = h;
-            vw[u] = wrapi(w0 - 1 + (tid >> 1) + 64 * u, x.w);
-        }
-    } else {
-        v0 = blockIdx.x * 128;
-#pragma unroll
-        for (int u = 0; u < 2; u++) decode(x, v0 + (tid >> 1) + 64 * u, vn[u], vd[u], vh[u], vw[u]);
-    }
+    const int cin = x.c, nchunk = cin >> 4;
+    int t = blockIdx.x;
+    const int w0 = (t % geo.tw) * 8;
+    t /= geo.tw;
+    const int h0 = (t % geo.th) * 16;
+    t /= geo.th;
+    const int z0 = (t % geo.tz) * geo.dz, n = t / geo.tz;
+    const int nq = min(geo.dz, x.d - z0);  // output planes of this tile
+    const int npl = nq + 2, nst = nchunk * npl;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(Cfg::kCols));
+                     "r"(geo.cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0)
-        for (int s = 0; s < S; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + s)));
+        for (int s = 0; s < kZmA; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + s)));
 
-    // stage `chunk` (units chunk*KU ..) into ring slot `s`
-    auto load = [&](int chunk, int s) {
-        unsigned char *As = A + (size_t)s * Cfg::A_BYTES, *Bs = B + (size_t)s * Cfg::B_BYTES;
+    // this thread's copies of a plane: chunk e = tid + 128 u is group e & 1 of voxel e >> 1
+    int src[3];
 #pragma unroll
-        for (int j = 0; j < Cfg::KU; j++) {
-            const int un = chunk * Cfg::KU + j;
-            if (un >= nu) break;
-            int dz, dy, dx0, cb;  // the unit's row (and tap) and channel block
-            if constexpr (ROW) {
-                const int rr = un / kpt;
-                cb = un - rr * kpt;
-                dz = rr / 3 - 1; dy = rr % 3 - 1; dx0 = 0;
-            } else {
-                const int tap = un / kpt;
-                cb = un - tap * kpt;
-                dz = tap / 9 - 1; dy = (tap / 3) % 3 - 1; dx0 = tap % 3 - 1;
-            }
+    for (int u = 0; u < 3; u++) {
+        const int hv = min((tid + 128 * u) >> 1, kZmVox - 1);
+        src[u] = (wrapn(h0 - 1 + hv / 10, x.h) * x.w + wrapn(w0 - 1 + hv % 10, x.w)) * x.ld + (tid & 1) * 8;
+    }
+    const int zstride = x.h * x.w * x.ld;
+    const bf16 *xn = x.p + (long long)n * x.d * zstride;
+    auto load_a = [&](int st) {
+        const int c = st / npl, r = st - c * npl;
+        const bf16 *p = xn + (long long)wrapn(z0 - 1 + r, x.d) * zstride + c * 16;
+        unsigned char *As = A + (size_t)(st % kZmA) * kZmPlane;
 #pragma unroll
-            for (int u = 0; u < (ROW ? 3 : 2); u++) {
-                const int vv = (tid >> 1) + 64 * u;  // A row of this copy
-                if (ROW && vv >= Cfg::VOX) break;
-                const bf16 *src = x.p +
-                                  (long long)vox(x, vn[u], wrapi(vd[u] + dz, x.d), wrapi(vh[u] + dy, x.h),
-                                                 ROW ? vw[u] : wrapi(vw[u] + dx0, x.w)) * x.ld + cb * 16 + ag * 8;
-                cpa16(As + (size_t)j * Cfg::A_UNIT + ((size_t)ag * Cfg::VOX + vv) * 16, src);
-            }
-            for (int e = tid; e < Cfg::TAPS * 2 * N; e += 128) {
-                const int t3 = e / (2 * N), r2 = e - t3 * 2 * N, g = r2 / N, o = r2 - g * N;
-                const int tap = ROW ? (dz + 1) * 9 + (dy + 1) * 3 + t3 : (dz + 1) * 9 + (dy + 1) * 3 + dx0 + 1;
-                cpa16(Bs + (size_t)j * Cfg::B_UNIT + ((size_t)(t3 * 2 + g) * N + o) * 16,
-                      wt + ((long long)tap * N + o) * cin + cb * 16 + g * 8);
-            }
+        for (int u = 0; u < 3; u++) {
+            const int e = tid + 128 * u;
+            if (e < 2 * kZmVox) cpa16(As + (e & 1) * (kZmVox * 16) + (e >> 1) * 16, p + src[u]);
+        }
+    };
+    // weights of chunk c: [dy, dx][group][dz = +1, 0, -1][cout][16 B]
+    auto load_b = [&](int c) {
+        unsigned char *Bs = B + (size_t)(c % geo.nb) * kB;
+        for (int e = tid; e < 54 * N; e += 128) {
+            const int g = e & 1, o = (e >> 1) % N, tap = (e >> 1) / N;  // tap = 9 dz + 3 dy + dx
+            const int dzi = tap / 9, t9 = tap - 9 * dzi;
+            cpa16(Bs + (((t9 * 2 + g) * 3 + 2 - dzi) * N + o) * 16, wt + ((long long)tap * N + o) * cin + c * 16 + g * 8);
         }
     };
     auto commit_group = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
+    load_b(0);
 #pragma unroll 1
-    for (int p = 0; p < S - 1; p++) {
-        if (p < nK) load(p, p);
+    for (int p = 0; p < kZmA - 1; p++) {
+        if (p < nst) {
+            if (p && p % npl == 0 && geo.nb > 1) load_b(p / npl);
+            load_a(p);
+        }
         commit_group();
     }
     __syncthreads();  // barrier inits and the TMEM address are visible
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = *reinterpret_cast<volatile unsigned *>(tmem_slot);
-    const uint32_t idesc = umma_idesc_bf16(N);
+    // the accumulators start at zero
+    for (int c0 = 0; c0 < nq * N; c0 += 16)
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+                tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0), "r"(0));
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     bool ok = true;
 #pragma unroll 1
-    for (int k = 0; k < nK; k++) {
-        const int s = k % S;
-        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");  // stage k has landed
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // visible to the tensor core
+    for (int st = 0; st < nst; st++) {
+        const int c = st / npl, r = st - c * npl;
+        if (st && r == 0 && geo.nb == 1) {
+            // one weight buffer: the MMAs of the chunk before have to be done
+            const bool done = mbar_wait(mbar + (st - 1) % kZmA, ((st - 1) / kZmA) & 1);
+            if (__syncthreads_or(!done)) {
+                ok = false;
+                break;
+            }
+            load_b(c);
+            commit_group();
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kZmA - 2) : "memory");  // stage st has landed
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor core
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned as = smem_u32(A + (size_t)s * Cfg::A_BYTES), bs = smem_u32(B + (size_t)s * Cfg::B_BYTES);
+            const unsigned as = smem_u32(A + (size_t)(st % kZmA) * kZmPlane), bs = smem_u32(B + (size_t)(c % geo.nb) * kB);
+            // output planes lo .. hi (tile-local) of input plane r - 1
+            const int lo = max(0, r - 2), hi = min(nq - 1, r), b0 = lo - (r - 2);
+            const int nblk = hi - lo + 1, per = 3 * N <= 256 ? nblk : 1;
+            const uint32_t idesc = umma_idesc_bf16(per * N);
 #pragma unroll 1
-            for (int j = 0; j < Cfg::KU; j++) {
-                const int un = k * Cfg::KU + j;
-                if (un >= nu) break;
-#pragma unroll
-                for (int t3 = 0; t3 < Cfg::TAPS; t3++) {
-                    // ROW: tap dx = t3 - 1 reads the halo row shifted by t3 voxels
-                    const uint64_t ad = umma_desc(as + j * Cfg::A_UNIT + t3 * 16, Cfg::VOX * 16, 128);
-                    const uint64_t bd = umma_desc(bs + j * Cfg::B_UNIT + t3 * 2 * N * 16, N * 16, 128);
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
-                        ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"((un > 0 || t3 > 0) ? 1 : 0), "r"(0));
-                }
+            for (int t9 = 0; t9 < 9; t9++) {
+                const uint64_t ad = umma_desc(as + ((t9 / 3) * 10 + t9 % 3) * 16, kZmVox * 16, 160);
+                for (int b = 0; b < nblk; b += per)
+                    umma_bf16(tmem + (lo + b) * N, ad, umma_desc(bs + (t9 * 6 + b0 + b) * N * 16, 3 * N * 16, 128), idesc);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(smem_u32(mbar + s)) : "memory");
+                         ::"r"(smem_u32(mbar + st % kZmA)) : "memory");
         }
-        const int nk = k + S - 1;  // the stage to fill next, in the slot stage k-1 used
-        if (nk < nK) {
-            if (k >= 1) {
-                const bool done = mbar_wait(mbar + nk % S, ((k - 1) / S) & 1);
+        const int nx = st + kZmA - 1;  // the stage to fill next, in the slot stage st-1 used
+        if (nx < nst) {
+            if (st >= 1) {
+                const bool done = mbar_wait(mbar + nx % kZmA, ((st - 1) / kZmA) & 1);
                 if (__syncthreads_or(!done)) {
                     ok = false;
                     break;
                 }
             }
-            load(nk, nk % S);
+            if (nx % npl == 0 && geo.nb > 1) load_b(nx / npl);
+            load_a(nx);
         }
         commit_group();
     }
     bool done = false;
-    if (ok) done = mbar_wait(mbar + (nK - 1) % S, ((nK - 1) / S) & 1);
+    if (ok) done = mbar_wait(mbar + (nst - 1) % kZmA, ((nst - 1) / kZmA) & 1);
     if (__syncthreads_or(!done)) {
         done = false;
         if (tid == 0) atomicExch(err, 1);
@@ -335,33 +343,40 @@ __global__ void __launch_bounds__(128) k_conv3_tcg(Act x, const bf16 *__restrict
     asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (done) {
-        const long long v = v0 + tid;  // TMEM lane = tile row = voxel
+        // TMEM lane = tile row = voxel (h0 + tid / 8, w0 + tid % 8)
+        const int h = h0 + (tid >> 3), w = w0 + (tid & 7);
+        const bool in = h < x.h && w < x.w;
+        for (int q = 0; q < nq; q++) {
+            bf16 *dst = y.p + ((((long long)n * x.d + z0 + q) * x.h + h) * x.w + w) * y.ld;
 #pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            unsigned r[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                : "r"(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            __nv_bfloat162 o2[8];
+            for (int c0 = 0; c0 < N; c0 += 16) {
+                unsigned v[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                    : "r"(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(q * N + c0)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                __nv_bfloat162 o2[8];
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                float a = __uint_as_float(r[2 * q]) + (bias ? bias[c0 + 2 * q] : 0.f);
-                float b = __uint_as_float(r[2 * q + 1]) + (bias ? bias[c0 + 2 * q + 1] : 0.f);
-                if (relu) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
-                o2[q] = __floats2bfloat162_rn(a, b);
+                for (int m = 0; m < 8; m++) {
+                    float a = __uint_as_float(v[2 * m]) + (bias ? bias[c0 + 2 * m] : 0.f);
+                    float b = __uint_as_float(v[2 * m + 1]) + (bias ? bias[c0 + 2 * m + 1] : 0.f);
+                    if (relu) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
+                    o2[m] = __floats2bfloat162_rn(a, b);
+                }
+                if (in) {
+                    uint4 *d4 = reinterpret_cast<uint4 *>(dst + c0);
+                    d4[0] = *reinterpret_cast<uint4 *>(&o2[0]);
+                    d4[1] = *reinterpret_cast<uint4 *>(&o2[4]);
+                }
             }
-            uint4 *dst = reinterpret_cast<uint4 *>(y.p + v * y.ld + c0);
-            dst[0] = *reinterpret_cast<uint4 *>(&o2[0]);
-            dst[1] = *reinterpret_cast<uint4 *>(&o2[4]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::kCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(geo.cols));
 }
 
 int *tc_err_flag() {
@@ -370,57 +385,50 @@ int *tc_err_flag() {
     return flag;
 }
 
-// the tcgen05 path: whole 128-voxel tiles, 16-byte aligned channel rows, and
-// an output width the kernel is instantiated for
+// the tcgen05 path: 16-byte aligned channel rows and an output width the
+// kernel is instantiated for
 bool tc_eligible(const Act &x, const Act &y) {
     static const bool off = getenv("BBMG_NO_TCGEN05") != nullptr;
-    if (off || x.nvox % 128 || x.c % 16) return false;
+    if (off || x.c % 16) return false;
     if (y.c != 16 && y.c != 32 && y.c != 48 && y.c != 64 && y.c != 96 && y.c != 128 && y.c != 192) return false;
     return !(x.ld % 8 || y.ld % 8 || (reinterpret_cast<uintptr_t>(x.p) & 15) || (reinterpret_cast<uintptr_t>(y.p) & 15));
 }
 
-template <int N, bool ROW, int S>
-int launch_conv_tc_t(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
-    using Cfg = TgCfg<N, ROW, S>;
+template <int N>
+int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
+    constexpr int kFixed = 128 + kZmA * kZmPlane, kB = 27 * N * 32;
+    constexpr int kTwoPerSm = 112 * 1024, kMost = 226 * 1024;
+    static_assert(kFixed + kB <= kMost, "one weight buffer has to fit");
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(k_conv3_tcg<N, ROW, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM) !=
-            cudaSuccess)
+        if (cudaFuncSetAttribute(k_conv3_zm<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess)
             return BBMG_CUDA;
         attr = true;
     }
     int *err = tc_err_flag();
     if (!err) return BBMG_NO_MEMORY;
-    k_conv3_tcg<N, ROW, S><<<x.nvox / 128, 128, Cfg::SMEM, s>>>(x, wt, bias, y, relu, err);
+    ZmGeo g;
+    g.tw = (x.w + 7) / 8;
+    g.th = (x.h + 15) / 16;
+    // output planes per tile: as many as 256 TMEM columns hold (two CTAs share
+    // an SM's 512), fewer where that would leave SMs idle
+    const long long cols = (long long)g.tw * g.th * x.n;
+    g.dz = min(x.d, max(1, 256 / N));
+    while (g.dz > 1 && cols * ((x.d + g.dz - 1) / g.dz) < 2 * 148) g.dz = (g.dz + 1) / 2;
+    g.tz = (x.d + g.dz - 1) / g.dz;
+    for (g.cols = 32; g.cols < g.dz * N;) g.cols *= 2;
+    // two weight buffers where two CTAs per SM still fit with them, or where
+    // only one fits anyway
+    const bool two = kFixed + 2 * kB <= kTwoPerSm || (kFixed + kB > kTwoPerSm && kFixed + 2 * kB <= kMost);
+    g.nb = x.c > 16 && two ? 2 : 1;
+    const long long grid = cols * g.tz;
+    if (grid >= (1LL << 31)) return BBMG_BAD_ARGS;
+    k_conv3_zm<N><<<(unsigned)grid, 128, kFixed + g.nb * kB, s>>>(x, wt, bias, y, relu, g, err);
     return done(cudaGetLastError());
-}
-
-// ring depth S (BBMG_TC_STAGES = 2, 3 or 4): with 2 stages a CTA needs half
-// the shared memory of 4 and about twice as many CTAs share an SM; measured
-// at 128^3 the forward pass took 3.66 ms with 2 stages, 3.72 with 3, 3.79
-// with 4
-template <int N, bool ROW>
-int launch_conv_tc_s(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
-    static int st = -1;
-    if (st < 0) {
-        const char *e = getenv("BBMG_TC_STAGES");
-        st = e ? atoi(e) : 2;
-    }
-    if (st == 2) return launch_conv_tc_t<N, ROW, 2>(x, wt, bias, y, relu, s);
-    if (st == 3) return launch_conv_tc_t<N, ROW, 3>(x, wt, bias, y, relu, s);
-    return launch_conv_tc_t<N, ROW, 4>(x, wt, bias, y, relu, s);
-}
-
-template <int N>
-int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
-    static const bool no_rows = getenv("BBMG_NO_TC_ROWS") != nullptr;
-    return (x.w % 128 == 0 && !no_rows) ? launch_conv_tc_s<N, true>(x, wt, bias, y, relu, s)
-                                        : launch_conv_tc_s<N, false>(x, wt, bias, y, relu, s);
 }
 
 int launch_conv(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
     const int blocks = (x.nvox + 63) / 64;
-    // whole 128-voxel tiles: the tcgen05 kernel
     if (tc_eligible(x, y)) {
         switch (y.c) {
         case 16: return launch_conv_tc<16>(x, wt, bias, y, relu, s);

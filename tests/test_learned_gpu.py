@@ -454,3 +454,24 @@ def test_network_with_tcgen05_rows_matches_oracle():
     ref = U.forward(net.params.cpu().double(), x, round_bf16=True).reshape(-1)
     rel = float((out - ref).norm() / ref.norm())
     assert rel < 3e-2, rel
+
+
+@pytest.mark.parametrize("cin,cout,shape", [
+    # one voxel per direction, sizes under and just over a tile of 8 x 16 voxels, odd sizes, two batches,
+    # plane counts around the tile's (16 planes at 16 channels, one at 192), one and several input chunks
+    (16, 16, (1, 1, 1, 1)), (16, 16, (1, 17, 17, 9)), (32, 16, (2, 3, 15, 7)), (48, 64, (1, 5, 16, 8)),
+    (16, 192, (1, 2, 18, 5)), (128, 128, (1, 3, 2, 2)), (96, 32, (1, 9, 5, 24))])
+def test_convolution_tile_edges(L, cin, cout, shape):
+    """Convolutions on grids that are not whole tiles, against the oracle."""
+    rng = np.random.default_rng(7 * cin + cout)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    wt_ = bf(rng.standard_normal((27, cin, cout)) / np.sqrt(27 * cin))
+    b = torch.as_tensor(rng.standard_normal(cout) * 0.1, dtype=torch.float32)
+    xg = to_cl(x)
+    yg = torch.full((n * d * h * w, cout), float("nan"), dtype=torch.bfloat16, device="cuda")
+    wt, _ = packed(L, wt_.numpy())
+    bg = b.cuda()
+    assert L.nn_conv3(C.byref(act(xg, shape)), P(wt), P(bg), C.byref(act(yg, shape)), 1, None) == 0
+    assert L.nn_tc_error() == 0
+    close_bf16(from_cl(yg, shape), torch.relu(U.conv3(x, wt_, b.double())))
