@@ -81,15 +81,13 @@ struct bbmg_handle {
     std::vector<Level> lv;  // 1-based: lv[0] unused
     // coarsest dense problem
     int np = 0, lu_info = 0, npinned = 0;
-    // coarse tail of the V-cycle in one cluster launch from level tail_n0
-    // (0: every level runs pass by pass)
-    int tail_n0 = 0;
-    bool tail_off = false;        // cluster launch unavailable or not capturable: pass by pass
-    int tail_blocks[2] = {0, 0};  // cluster size per precision (0 = not sized yet)
-    size_t tail_smem_b = 0;
-    int tail_mat_in_smem = 0;
+    // coarse levels of the V-cycle in one cluster launch, per precision (0 FP64,
+    // 1 FP32): from level tail_n0 (0: every level runs pass by pass)
+    int tail_n0[2] = {0, 0};
+    bool tail_off = false;  // cluster launch not capturable: pass by pass
+    int tail_blocks[2] = {0, 0};
     double *OP = nullptr, *LU = nullptr;
-    int *piv = nullptr, *pinned = nullptr, *d_info = nullptr, *d_flag = nullptr;
+    int *piv = nullptr, *perm = nullptr, *pinned = nullptr, *d_info = nullptr, *d_flag = nullptr;
     // Krylov / outer iteration vectors (level-1 layout)
     double *sol = nullptr, *pp = nullptr, *pp2 = nullptr, *Ap = nullptr;  // pp/pp2 alternate per iteration
     double *x2 = nullptr;  // second solution buffer of the mixed defect correction (alternates with lv[1].v)
@@ -198,49 +196,62 @@ void drop_graphs(bbmg_handle *h) {
 // V-cycle (bbmg_class.f90:732-776), recursive over levels
 template <typename T> struct PrecIdx { static constexpr int value = sizeof(T) == 8 ? 0 : 1; };
 
-// cycle(n) for n >= tail_n0 as one cooperative launch; returns BBMG_NOT_SETUP
-// (nothing launched) when the levels do not qualify
+// sizes of the fused levels n..nlvl for a cluster of `blocks`
+template <typename T>
+bool plan_tail(bbmg_handle *h, int n, int blocks, TailArgs<T> *A, size_t *smem) {
+    Lay lay[kTailMax];
+    bool fuse[kTailMax];
+    const int cnt = h->nlvl - n + 1;
+    if (cnt > kTailMax) return false;
+    for (int m = 0; m < cnt; m++) {
+        lay[m] = h->lv[n + m].L;
+        fuse[m] = h->lv[n + m].fuse;
+    }
+    return tail_plan<T>(lay, fuse, cnt, h->lv[n].npt, h->np, h->prm.use_direct_solve != 0, blocks, A, smem);
+}
+
+// the first level from which the cycle can run in one cluster launch
+template <typename T>
+void choose_tail(bbmg_handle *h) {
+    constexpr int pi = PrecIdx<T>::value;
+    long long most = kTailCells;
+    if (const char *env = getenv("BBMG_TAIL_CELLS")) most = atoll(env);
+    for (int n = 1; h->prm.ncycle == 1 && n < h->nlvl; n++) {
+        const Lay &L = h->lv[n].L;
+        if ((long long)L.nx * L.ny * L.nz > most) continue;
+        TailArgs<T> A{};
+        size_t smem = 0;
+        for (int blocks = kTailClusterMax; blocks >= 8; blocks /= 2) {
+            if (!plan_tail<T>(h, n, blocks, &A, &smem) || !tail_fits<T>(blocks)) continue;
+            h->tail_n0[pi] = n;
+            h->tail_blocks[pi] = blocks;
+            return;
+        }
+    }
+}
+
+// cycle(n) for n = tail_n0 as one cluster launch
 template <typename T>
 int vcycle_tail(bbmg_handle *h, int n) {
     using P = LvlPtr<T>;
+    constexpr int pi = PrecIdx<T>::value;
     TailArgs<T> A{};
-    A.n = h->nlvl - n + 1;
-    if (A.n > kTailMax || A.n < 2) return BBMG_NOT_SETUP;
+    size_t smem = 0;
+    if (!plan_tail<T>(h, n, h->tail_blocks[pi], &A, &smem)) return fail(h, BBMG_CUDA, "coarse levels do not fit");
     for (int m = n; m <= h->nlvl; m++) {
         Level &l = h->lv[m];
-        if (l.npt != 27 || !l.fuse) return BBMG_NOT_SETUP;
         TailLvl<T> &t = A.lv[m - n];
-        t.L = l.L;
-        for (int q = 0; q < 27; q++) {
-            t.off[0].o[q] = l.nb.off[0][q];
-            t.off[1].o[q] = l.nb.off[1][q];
-        }
         t.opr = P::opr(l);
         t.v = P::v(l);
         t.f = P::f(l);
-        t.r = P::r(l);
         t.c2f = m < h->nlvl ? P::c2f(l) : nullptr;
     }
-    A.split = A.n - 1;
-    for (int m = 0; m < A.n - 1; m++) {
-        const Lay &L = A.lv[m].L;
-        if ((long long)L.nx * L.ny * L.nz <= kTailBlockCells) { A.split = m; break; }
-    }
-    if (const char *env = getenv("BBMG_TAIL_SPLIT")) A.split = std::max(0, std::min(A.n - 1, atoi(env)));
     A.pre = h->prm.relax_pre;
     A.post = h->prm.relax_post;
-    A.direct = h->prm.use_direct_solve;
-    A.mat_in_smem = h->tail_mat_in_smem;
     A.LU = h->LU;
-    A.piv = h->piv;
+    A.perm = h->perm;
     A.pinned = h->pinned;
-    int &blocks = h->tail_blocks[PrecIdx<T>::value];
-    if (!blocks && tail_grid<T>(h->tail_smem_b, &blocks) != cudaSuccess) {
-        cudaGetLastError();
-        h->tail_off = true;  // no cluster of 8 fits: the levels run pass by pass
-        return BBMG_NOT_SETUP;
-    }
-    CU(h, launch_vtail<T>(A, blocks, h->tail_smem_b, h->stream));
+    CU(h, launch_vtail<T>(A, h->lv[n].npt, h->tail_blocks[pi], smem, h->stream));
     return BBMG_OK;
 }
 
@@ -248,14 +259,11 @@ template <typename T>
 int vcycle(bbmg_handle *h, int n) {
     using P = LvlPtr<T>;
     cudaStream_t s = h->stream;
-    if (n == h->tail_n0 && !h->tail_off && h->prm.ncycle == 1) {
-        int st = vcycle_tail<T>(h, n);
-        if (st != BBMG_NOT_SETUP) return st;
-    }
+    if (n == h->tail_n0[PrecIdx<T>::value] && !h->tail_off) return vcycle_tail<T>(h, n);
     Level &l = h->lv[n];
     if (n == h->nlvl) {
         if (h->prm.use_direct_solve) {
-            CU(h, launch_coarse_solve<T>(l.L, h->LU, h->piv, h->pinned, P::f(l), P::v(l), s));
+            CU(h, launch_coarse_solve<T>(l.L, h->LU, h->perm, h->pinned, P::f(l), P::v(l), s));
         } else {
             CU(h, launch_relax_sweeps<T>(l.L, l.nb, l.npt, l.fuse, P::opr(l), P::v(l), P::f(l), 1,
                                          h->prm.relax_pre + h->prm.relax_post, s));
@@ -340,7 +348,7 @@ int get_graph(bbmg_handle *h, int mode, int par, cudaGraphExec_t *out) {
     CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int st = record_iteration(h, mode, par);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-    if ((st || e != cudaSuccess) && h->tail_n0 && !h->tail_off) {
+    if ((st || e != cudaSuccess) && (h->tail_n0[0] || h->tail_n0[1]) && !h->tail_off) {
         // a cluster launch that cannot be captured here: record the coarse
         // levels pass by pass instead
         if (g) cudaGraphDestroy(g);
@@ -413,7 +421,7 @@ int bbmg_destroy(bbmg_handle *h) {
         dfree(l.v); dfree(l.f); dfree(l.r);
         dfree(l.oprS32); dfree(l.c2f32); dfree(l.v32); dfree(l.f32); dfree(l.r32);
     }
-    dfree(h->OP); dfree(h->LU); dfree(h->piv); dfree(h->pinned); dfree(h->d_info); dfree(h->d_flag);
+    dfree(h->OP); dfree(h->LU); dfree(h->piv); dfree(h->perm); dfree(h->pinned); dfree(h->d_info); dfree(h->d_flag);
     dfree(h->sol); dfree(h->pp); dfree(h->pp2); dfree(h->Ap); dfree(h->x2); dfree(h->b1); dfree(h->sc); dfree(h->part);
     dfree(h->z1); dfree(h->zz);
     dfree(h->dscal);
@@ -525,7 +533,7 @@ int bbmg_create(const bbmg_grid *grid, const bbmg_params *params, bbmg_handle **
     }
     const Lay &L1 = h->lv[1].L;
     if ((st = dalloc(h, &h->OP, (size_t)h->np * h->np)) || (st = dalloc(h, &h->LU, (size_t)h->np * h->np)) ||
-        (st = dalloc(h, &h->piv, (size_t)h->np)) || (st = dalloc(h, &h->pinned, (size_t)h->np)) ||
+        (st = dalloc(h, &h->piv, (size_t)h->np)) || (st = dalloc(h, &h->perm, (size_t)h->np)) || (st = dalloc(h, &h->pinned, (size_t)h->np)) ||
         (st = dalloc(h, &h->d_info, 1)) || (st = dalloc(h, &h->d_flag, 1)) ||
         (st = dalloc(h, &h->part, 2 * (size_t)kRedBlocks)) ||
         (st = dalloc(h, &h->dscal, kScalN)) || (st = dalloc(h, &h->sc, 1)))
@@ -537,20 +545,8 @@ int bbmg_create(const bbmg_grid *grid, const bbmg_params *params, bbmg_handle **
             (st = dalloc(h, &h->b1, (size_t)L1.plane)))
             return bail(st);
     }
-    {
-        // the coarse tail: the first level >= 2 at or below tail_cells cells
-        // from which every level can be fused (27-point, periodic sizes even)
-        long long tail_cells = kTailCells;
-        if (const char *env = getenv("BBMG_TAIL_CELLS")) tail_cells = atoll(env);
-        for (int n = 2; prm.ncycle == 1 && tail_cells > 0 && n < h->nlvl; n++) {
-            const Lay &L = h->lv[n].L;
-            if ((long long)L.nx * L.ny * L.nz > tail_cells || h->nlvl - n + 1 > kTailMax) continue;
-            bool ok = true;
-            for (int m = n; m <= h->nlvl; m++) ok = ok && h->lv[m].fuse;
-            if (ok) { h->tail_n0 = n; break; }
-        }
-        if (h->tail_n0) h->tail_smem_b = tail_smem(h->np, &h->tail_mat_in_smem);
-    }
+    choose_tail<double>(h);
+    if (mixed) choose_tail<float>(h);
     if (cudaMallocHost((void **)&h->h_scal, kScalN * sizeof(double)) != cudaSuccess) return bail(fail(h, BBMG_NO_MEMORY, "pinned host"));
     if (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
         return bail(fail(h, BBMG_CUDA, "events"));
@@ -703,7 +699,7 @@ int bbmg_setup(bbmg_handle *h, int nst, const int *stc, const double *opr) {
         CU(h, setup_operator(F.L, C.L, F.opr27, F.c2f, C.f2c, F.oprc2f, C.opr27, fmask, s, mixed ? C.oprS32 : nullptr));
     }
     // dense coarsest problem (bbmg_class.f90:961, 1307-1385)
-    CU(h, setup_direct(h->lv[h->nlvl].L, h->lv[h->nlvl].opr27, h->OP, h->LU, h->piv, h->pinned, h->d_info, s));
+    CU(h, setup_direct(h->lv[h->nlvl].L, h->lv[h->nlvl].opr27, h->OP, h->LU, h->piv, h->perm, h->pinned, h->d_info, s));
     // solve-phase operator planes: a 7-point level-1 operator that is exactly
     // symmetric is stored as 4 planes (D, E, N, T), otherwise as 7; coarse
     // levels keep the 27 planes
@@ -1105,7 +1101,7 @@ static int debug_step_t(bbmg_handle *h, int step, int n, int arg) {
     }
     case BBMG_STEP_DIRECT: {
         Level &c = h->lv[h->nlvl];
-        CU(h, launch_coarse_solve<T>(c.L, h->LU, h->piv, h->pinned, P::f(c), P::v(c), s));
+        CU(h, launch_coarse_solve<T>(c.L, h->LU, h->perm, h->pinned, P::f(c), P::v(c), s));
         break;
     }
     default: return fail(h, BBMG_BAD_ARGS, "unknown step %d", step);

@@ -860,18 +860,41 @@ __device__ __forceinline__ void lu_block(double *A, int n, int *__restrict__ piv
     if (tid == 0) *info_out = s_info;
 }
 
-__global__ void k_lu(double *__restrict__ A, int n, int *__restrict__ piv, int *__restrict__ pinned,
+constexpr int kLuMax = 4096;  // most unknowns of a direct solve
+
+// perm: the row permutation that the successive swaps of piv add up to, so
+// that a solve gathers its right-hand side in one pass; pm holds n ints.
+__device__ __forceinline__ void lu_perm(const int *piv, int n, int *__restrict__ perm, int *pm, int *ps) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        pm[i] = i;
+        ps[i] = piv[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int j = 0; j < n; j++) {
+            const int p = ps[j], t = pm[j];
+            pm[j] = pm[p];
+            pm[p] = t;
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = pm[i];
+}
+
+__global__ void k_lu(double *__restrict__ A, int n, int *piv, int *__restrict__ perm, int *__restrict__ pinned,
                      int *__restrict__ info_out) {
     __shared__ double sval[1024];
     __shared__ int sidx[1024];
     __shared__ int s_info;
+    __shared__ int pm[2 * kLuMax];
     lu_block(A, n, piv, pinned, info_out, sval, sidx, s_info);
+    if (n <= kLuMax) lu_perm(piv, n, perm, pm, pm + n);
 }
 
 // The same factorisation with the matrix held in shared memory (n*n*8 bytes
 // plus blockDim.x * 12): the per-column barriers then wait on shared-memory
 // traffic instead of global-memory round trips.
-__global__ void k_lu_smem(double *__restrict__ A, int n, int *__restrict__ piv, int *__restrict__ pinned,
+__global__ void k_lu_smem(double *__restrict__ A, int n, int *piv, int *__restrict__ perm, int *__restrict__ pinned,
                           int *__restrict__ info_out) {
     extern __shared__ __align__(16) unsigned char lu_sm[];
     double *M = reinterpret_cast<double *>(lu_sm);
@@ -884,6 +907,7 @@ __global__ void k_lu_smem(double *__restrict__ A, int n, int *__restrict__ piv, 
     lu_block(M, n, piv, pinned, info_out, sval, sidx, s_info);
     __syncthreads();
     for (long long e = threadIdx.x; e < nn; e += blockDim.x) A[e] = M[e];
+    lu_perm(piv, n, perm, reinterpret_cast<int *>(M), reinterpret_cast<int *>(M) + n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1070,8 +1094,8 @@ cudaError_t check_symmetric7(const Lay &L, const double *opr, int *flag, cudaStr
     return cudaSuccess;
 }
 
-cudaError_t setup_direct(const Lay &L, const double *opr, double *OP, double *LU, int *piv, int *pinned, int *info,
-                         cudaStream_t s) {
+cudaError_t setup_direct(const Lay &L, const double *opr, double *OP, double *LU, int *piv, int *perm, int *pinned,
+                         int *info, cudaStream_t s) {
     int np = L.nx * L.ny * L.nz;
     k_dense_operator<<<(np + 127) / 128, 128, 0, s>>>(L, opr, OP);
     BB_LAUNCH_CHECK();
@@ -1086,9 +1110,9 @@ cudaError_t setup_direct(const Lay &L, const double *opr, double *OP, double *LU
             if (e != cudaSuccess) return e;
             attr = true;
         }
-        k_lu_smem<<<1, kLuThreads, lu_smem, s>>>(LU, np, piv, pinned, info);
+        k_lu_smem<<<1, kLuThreads, lu_smem, s>>>(LU, np, piv, perm, pinned, info);
     } else {
-        k_lu<<<1, 1024, 0, s>>>(LU, np, piv, pinned, info);
+        k_lu<<<1, 1024, 0, s>>>(LU, np, piv, perm, pinned, info);
     }
     BB_LAUNCH_CHECK();
     return cudaSuccess;

@@ -32,10 +32,13 @@ cudaError_t fill_overlap_oprc2f(const Lay &F, double *oprc2f, cudaStream_t s);
 cudaError_t setup_solve_planes(const Lay &L, const double *opr, int npt, const int *slots, double *oprS,
                                float *oprS32, cudaStream_t s);
 cudaError_t check_symmetric7(const Lay &L, const double *opr, int *flag, cudaStream_t s);
-cudaError_t setup_direct(const Lay &L, const double *opr, double *OP, double *LU, int *piv, int *pinned, int *info,
-                         cudaStream_t s);
+cudaError_t setup_direct(const Lay &L, const double *opr, double *OP, double *LU, int *piv, int *perm, int *pinned,
+                         int *info, cudaStream_t s);
 
 // solve.cu
+struct Off27 {
+    int o[27];
+};
 template <typename T>
 cudaError_t launch_relax(const Lay &L, const NbrOff &nb, int npt, bool fuse, const T *opr, T *v, const T *f, int dir,
                          cudaStream_t s, bool skip_first = false);
@@ -51,48 +54,58 @@ template <typename T>
 cudaError_t launch_restrict(const Lay &F, const Lay &C, const T *c2f, const T *rF, T *fC, T *vC, cudaStream_t s);
 template <typename T>
 cudaError_t launch_prolong(const Lay &F, const Lay &C, const T *c2f, const T *vC, T *vF, cudaStream_t s);
-constexpr size_t kCoarseSmem = 200 * 1024;  // factors of up to 158 unknowns stay on chip
+// vtail.cu: the coarsest solve; perm is the row permutation of the stored LU
+constexpr size_t kCoarseSmem = 200 * 1024;  // factors of up to 152 unknowns stay on chip
 cudaError_t coarse_solve_prepare();  // per device, before the first coarse solve
 template <typename T>
-cudaError_t launch_coarse_solve(const Lay &L, const double *LU, const int *piv, const int *pinned, const T *f, T *v,
+cudaError_t launch_coarse_solve(const Lay &L, const double *LU, const int *perm, const int *pinned, const T *f, T *v,
                                 cudaStream_t s);
 
-// the coarse tail of the V-cycle in one launch of one thread-block cluster
-// (levels n0..nlvl, 27-point operators, V-cycle only)
-struct Off27 {
-    int o[27];
-};
+// vtail.cu: levels n0..nlvl of the V-cycle in one launch of one thread-block
+// cluster (ncycle = 1; the first level may hold a 4- or 7-plane operator)
 template <typename T>
 struct TailLvl {
     Lay L;
-    Off27 off[2];          // neighbour offsets for even / odd x
-    const T *opr;          // 27 coefficient planes
-    T *v, *f, *r;
+    const T *opr;          // coefficient planes
+    T *v;                  // global v and f: the first level's are read and written
+    const T *f;
     const T *c2f;          // prolongation weights of this level (to the next coarser one)
+    int fuse;              // periodic images may be written inside a colour
+    int single;            // inside block 0
+    int H;                 // k-planes per block
+    int PX, E0, PP;        // shared memory: row pitch, offset of the even x, plane pitch
+    int sv, sf, sr, sc;    // first elements of V, F, R and the coefficients (-1: in global memory)
+    int ncf;               // elements of F, of R and of one coefficient
+    float iH, inx, iny, ia, ib;  // reciprocals of H, nx, ny and of a colour's points per row and rows
 };
 constexpr int kTailMax = 8;            // levels in one launch (kernel parameters stay under 4 KB)
-constexpr int kTailThreads = 512;
+constexpr int kTailThreads = 256;
 constexpr int kTailClusterMax = 16;    // blocks of the cluster (non-portable size; 8 if refused)
-constexpr long long kTailCells = 512;  // first fused level: at most 8^3 cells.  Larger levels run
-                                       // faster as staged passes in the iteration's CUDA graph
-                                       // (measured: fused from 32^3 27.8 ms per 256^3 mixed solve,
-                                       // from 16^3 27.4, from 8^3 27.0)
-constexpr size_t kTailSmemMax = 100 * 1024;
-constexpr long long kTailBlockCells = 4096;  // levels this small run inside one block
+constexpr long long kTailCells = 36864;      // most cells of the first fused level
+constexpr long long kTailBlockCells = 4096;  // most cells of a block's slab
+constexpr long long kTailSingle = 1024;      // levels this small run inside block 0
+constexpr size_t kTailMatMax = 136 * 1024;   // LU factors held in shared memory
+constexpr size_t kTailSmemMax = 226 * 1024;
 template <typename T>
 struct TailArgs {
     TailLvl<T> lv[kTailMax];
     int n;                 // levels in lv; lv[n-1] is the coarsest
-    int split;             // levels >= split (when split < n-1) run inside one block
-    int pre, post, direct, mat_in_smem;
+    int split;             // levels below it are dealt out over the cluster
+    int pre, post, direct, np, mat_in_smem;
+    int solve_bytes, zeroed;  // shared memory: bytes of the coarsest solve, then values that start at zero
     const double *LU;
-    const int *piv, *pinned;
+    const int *perm, *pinned;
 };
-size_t tail_smem(int np, int *mat_in_smem);
+// sizes and shared-memory layout of the n levels lay[0..n) for a cluster of
+// `blocks`, the first with npt1 planes; false if they do not fit.  tail_fits:
+// the device can run it.
 template <typename T>
-cudaError_t tail_grid(size_t smem, int *blocks);
+bool tail_plan(const Lay *lay, const bool *fuse, int n, int npt1, int np, bool direct, int blocks, TailArgs<T> *A,
+               size_t *smem);
 template <typename T>
-cudaError_t launch_vtail(const TailArgs<T> &A, int blocks, size_t smem, cudaStream_t s);
+bool tail_fits(int blocks);
+template <typename T>
+cudaError_t launch_vtail(const TailArgs<T> &A, int npt1, int blocks, size_t smem, cudaStream_t s);
 // reductions (deterministic two-pass) into a device double
 constexpr int kRedBlocks = 1184;  // 8 blocks of 256 threads per SM on 148 SMs
 template <typename T>

@@ -16,7 +16,7 @@
 // hit the lines the aligned loads just brought in.
 #include <cstdlib>
 
-#include "setup.cuh"
+#include "ops.cuh"
 
 namespace bbmg {
 
@@ -25,64 +25,6 @@ static Off27 off_for(const NbrOff &nb, int par) {
     for (int q = 0; q < 27; q++) r.o[q] = nb.off[par][q];
     return r;
 }
-
-// Programmatic dependent launch: every solve-phase kernel lets the next kernel
-// in the stream start launching as soon as all of its own blocks are running,
-// then waits for its predecessor to finish (and its writes to be visible)
-// before touching memory.  Semantics stay those of plain stream order; only
-// the launch latency overlaps the previous kernel's tail.
-__device__ __forceinline__ void pdl_entry() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-// The two halves, for kernels that first read data no kernel of the solve
-// writes (the operator planes, written only by the setup, which ends with a
-// stream synchronisation): those loads may start before the wait, while the
-// predecessor (or the one before it, still running its own tail) finishes.
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// L2 prefetch of the line holding p (a hint; L2 is coherent, so it is safe
-// for any operand, also one the predecessor is still writing)
-__device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t shm, cudaStream_t s,
-                            Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = shm;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
-#define BB_CHECK_LAUNCH(call)                \
-    do {                                     \
-        cudaError_t e0_ = (call);            \
-        if (e0_ != cudaSuccess) return e0_;  \
-        cudaError_t e_ = cudaGetLastError(); \
-        if (e_ != cudaSuccess) return e_;    \
-    } while (0)
-
-template <typename T, bool EXACT> struct Ops;
-template <> struct Ops<double, true> {
-    __device__ static __forceinline__ double mac(double s, double a, double b) { return __dadd_rn(s, __dmul_rn(a, b)); }
-    __device__ static __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
-    __device__ static __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-    __device__ static __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
-};
-template <typename T> struct Ops<T, false> {
-    __device__ static __forceinline__ T mac(T s, T a, T b) { return fma(a, b, s); }
-    __device__ static __forceinline__ T add(T a, T b) { return a + b; }
-    __device__ static __forceinline__ T sub(T a, T b) { return a - b; }
-    __device__ static __forceinline__ T div(T a, T b) { return a / b; }
-};
-template <typename T> struct ExactOf { static constexpr bool value = sizeof(T) == 8; };
 
 // ---------------------------------------------------------------------------
 // launch geometry: x = chunks of a row, y = rows (grid-stride in both)
@@ -978,75 +920,6 @@ __global__ void __launch_bounds__(128) k_prolong_staged(Lay F, Lay C, const T *_
     }
 }
 
-// Coarsest level: gather f in lexicographic order, solve with the stored LU
-// (FP64 always), scatter into v (bbmg_class.f90:891-927).  One block; the
-// triangular solves run on one warp with the factors in shared memory when
-// they fit.
-template <typename T>
-__device__ __forceinline__ void coarse_solve_block(const Lay &L, const double *__restrict__ LU,
-                                                   const int *__restrict__ piv, const int *__restrict__ pinned,
-                                                   const T *__restrict__ f, T *__restrict__ v, int mat_in_smem,
-                                                   double *sm) {
-    const int np = L.nx * L.ny * L.nz;
-    double *x = sm;
-    const double *A = mat_in_smem ? sm + np : LU;
-    for (int ind = threadIdx.x; ind < np; ind += blockDim.x) {
-        int i = ind % L.nx, j = (ind / L.nx) % L.ny, k = ind / (L.nx * L.ny);
-        x[ind] = (double)f[L.idx(i, j, k)];
-    }
-    if (mat_in_smem)
-        for (long long e = threadIdx.x; e < (long long)np * np; e += blockDim.x) sm[np + e] = LU[e];
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        if (lane == 0)
-            for (int j = 0; j < np; j++) {
-                int p = piv[j];
-                if (p != j) { double t = x[j]; x[j] = x[p]; x[p] = t; }
-            }
-        __syncwarp();
-        for (int kk = 0; kk < np; kk++) {
-            double xk = x[kk];
-            if (xk != 0.0)
-                for (int i = kk + 1 + lane; i < np; i += 32)
-                    x[i] = __dsub_rn(x[i], __dmul_rn(xk, A[(long long)kk * np + i]));
-            __syncwarp();
-        }
-        for (int kk = np - 1; kk >= 0; kk--) {
-            if (pinned[kk]) {
-                if (lane == 0) x[kk] = 0.0;
-                __syncwarp();
-                continue;
-            }
-            double xk = x[kk];
-            if (xk != 0.0) {
-                xk = __ddiv_rn(xk, A[(long long)kk * np + kk]);
-                __syncwarp();
-                if (lane == 0) x[kk] = xk;
-                for (int i = lane; i < kk; i += 32)
-                    x[i] = __dsub_rn(x[i], __dmul_rn(xk, A[(long long)kk * np + i]));
-            }
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    for (int ind = threadIdx.x; ind < np; ind += blockDim.x) {
-        int i = ind % L.nx, j = (ind / L.nx) % L.ny, k = ind / (L.nx * L.ny);
-        T val = (T)x[ind];
-        v[L.idx(i, j, k)] = val;
-        if (on_periodic_face(L, i, j, k)) write_images(L, v, i, j, k, val);
-    }
-}
-
-template <typename T>
-__global__ void k_coarse_solve(Lay L, const double *__restrict__ LU, const int *__restrict__ piv,
-                               const int *__restrict__ pinned, const T *__restrict__ f, T *__restrict__ v,
-                               int mat_in_smem) {
-    pdl_entry();
-    extern __shared__ double sm[];
-    coarse_solve_block<T>(L, LU, piv, pinned, f, v, mat_in_smem, sm);
-}
-
 // ---------------------------------------------------------------------------
 // Deterministic reductions: a fixed grid per level, a fixed tree per block.
 template <int MODE>  // 0 = max with NaN propagation, 1 = sum
@@ -1884,8 +1757,9 @@ cudaError_t launch_relax_sweeps(const Lay &L, const NbrOff &nb, int npt, bool fu
             // the first colour of a sweep after the opposite sweep is the colour
             // that sweep ended with: the reference's update (rhs minus the
             // neighbours' sum, over the centre) reads only the other colours,
-            // so recomputing it gives the same bits and is skipped
-            cudaError_t e = launch_relax<T>(L, nb, npt, fuse, opr, v, f, dir, s, i > 0);
+            // so recomputing it gives the same bits and is skipped (with an odd
+            // periodic size only the all-odd colour has no cell at the wrap)
+            cudaError_t e = launch_relax<T>(L, nb, npt, fuse, opr, v, f, dir, s, i > 0 && (fuse || dir < 0));
             if (e != cudaSuccess) return e;
             dir = -dir;
         }
@@ -2019,24 +1893,6 @@ cudaError_t launch_prolong(const Lay &F, const Lay &C, const T *c2f, const T *vC
     const Geo g = geo_rows(F.nx, (long long)F.ny * F.nz);
     BB_CHECK_LAUNCH((launch_k(k_prolong<T>, g.grid, g.block, 0, s, F, C, c2f, vC, vF)));
     return cudaSuccess;
-}
-
-template <typename T>
-cudaError_t launch_coarse_solve(const Lay &L, const double *LU, const int *piv, const int *pinned, const T *f, T *v,
-                                cudaStream_t s) {
-    int np = L.nx * L.ny * L.nz;
-    size_t mat = (size_t)np * np * sizeof(double), vec = (size_t)np * sizeof(double);
-    int in_smem = (mat + vec) <= kCoarseSmem;
-    size_t shm = vec + (in_smem ? mat : 0);
-    BB_CHECK_LAUNCH((launch_k(k_coarse_solve<T>, dim3(1), dim3(256), shm, s, L, LU, piv, pinned, f, v, in_smem)));
-    return cudaSuccess;
-}
-
-cudaError_t coarse_solve_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(k_coarse_solve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kCoarseSmem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_coarse_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem);
 }
 
 template <typename T>
@@ -2191,182 +2047,6 @@ cudaError_t launch_defect_fused(const Lay &L, const NbrOff &nb, int npt, const d
     return cudaSuccess;
 }
 
-// ---------------------------------------------------------------------------
-// The coarse tail of the V-cycle in one launch.  On levels of at most a few
-// hundred thousand cells a colour pass, residual, restriction or prolongation
-// is a few microseconds of work but a full kernel launch (about 35 launches
-// per level and cycle).  This kernel runs cycle(n0) (bbmg_class.f90:732-776)
-// for every level n0..nlvl inside one thread-block cluster: the passes are
-// separated by the cluster's hardware barrier, whose release/acquire
-// semantics make each pass's global-memory writes visible to the next.  A
-// cluster is scheduled as a unit, so no block can wait on one that is not
-// running, and no barrier can outlive its kernel.  Each pass calls the same
-// per-point functions as the single-pass kernels, so FP64 results stay
-// bit-identical.
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// The passes of the tail, over the threads [tid, nth) of either the whole
-// cluster (CL: a cluster barrier after each pass) or block 0 alone.
-template <bool CL>
-__device__ __forceinline__ void pass_sync() {
-    if (CL) cluster_sync_all();
-    else __syncthreads();
-}
-
-// skip: leave out the first colour (the one the opposite sweep before ended
-// with; recomputing it gives the same bits).  The loop keeps its fixed start:
-// with a runtime start ptxas gave the tail kernel half the registers (64
-// against 127) and its passes ran ~40 % slower.
-template <bool CL, typename T>
-__device__ void tail_relax(const TailLvl<T> &l, int dir, int tid, int nth, bool skip) {
-    for (int c = 0; c < 8; c++) {
-        if (c == 0 && skip) continue;
-        const int col = dir > 0 ? c : 7 - c;  // colours 1..8 forward, 8..1 backward
-        const int px = col & 1, py = (col >> 1) & 1, pz = (col >> 2) & 1;
-        const Lay &L = l.L;
-        const int na = (L.nx - px + 1) >> 1, nb = (L.ny - py + 1) >> 1, nc = (L.nz - pz + 1) >> 1;
-        const int n = na * nb * nc;
-        if (n == 0) continue;
-        const long long hb = px ? 0 : L.B0;
-        for (int it = tid; it < n; it += nth) {
-            const int a = it % na, row = it / na;
-            const int j = py + 2 * (row % nb), k = pz + 2 * (row / nb);
-            gs_points<T, 27, 1>(L, l.off[px], l.opr, l.v, l.f, L.G + L.row(j, k) * L.P + hb + a, px, j, k, a, 1);
-        }
-        pass_sync<CL>();
-    }
-}
-
-// pre-smoothing, residual and restriction of level l into c (bbmg_class.f90:750-763)
-template <bool CL, typename T>
-__device__ void tail_down(const TailArgs<T> &A, const TailLvl<T> &l, const TailLvl<T> &c, int tid, int nth) {
-    int dir = 1;
-    for (int i = 0; i < A.pre; i++, dir = -dir) {
-        tail_relax<CL>(l, dir, tid, nth, i > 0);
-    }
-    const Lay &L = l.L;
-    for (int it = tid; it < L.nx * L.ny * L.nz; it += nth) {
-        const int i = it % L.nx, row = it / L.nx;
-        residual_point<T, 27>(L, l.off[0].o, l.off[1].o, l.opr, l.v, l.f, l.r, i, row % L.ny, row / L.ny);
-    }
-    pass_sync<CL>();
-    const Lay &C = c.L;
-    for (int it = tid; it < C.nx * C.ny * C.nz; it += nth) {
-        const int i = it % C.nx, row = it / C.nx;
-        restrict_point<T>(L, C, l.c2f, l.r, c.f, c.v, i, row % C.ny, row / C.ny);
-    }
-    pass_sync<CL>();
-}
-
-// prolongation + correction into l from c, post-smoothing (bbmg_class.f90:766-775)
-template <bool CL, typename T>
-__device__ void tail_up(const TailArgs<T> &A, const TailLvl<T> &l, const TailLvl<T> &c, int tid, int nth) {
-    const Lay &F = l.L;
-    for (int it = tid; it < F.nx * F.ny * F.nz; it += nth) {
-        const int i = it % F.nx, row = it / F.nx;
-        prolong_point<T>(F, c.L, l.c2f, c.v, l.v, i, row % F.ny, row / F.ny);
-    }
-    pass_sync<CL>();
-    int dir = (A.pre & 1) ? -1 : 1;
-    for (int i = 0; i < A.post; i++, dir = -dir) {
-        tail_relax<CL>(l, dir, tid, nth, i > 0);
-    }
-}
-
-// coarsest level (bbmg_class.f90:741-748): block 0 solves with the stored LU
-template <bool CL, typename T>
-__device__ void tail_coarsest(const TailArgs<T> &A, double *sm, int tid, int nth) {
-    const TailLvl<T> &lc = A.lv[A.n - 1];
-    if (A.direct) {
-        if (blockIdx.x == 0) coarse_solve_block<T>(lc.L, A.LU, A.piv, A.pinned, lc.f, lc.v, A.mat_in_smem, sm);
-        pass_sync<CL>();
-        return;
-    }
-    int dir = 1;
-    for (int i = 0; i < A.pre + A.post; i++, dir = -dir) {
-        tail_relax<CL>(lc, dir, tid, nth, i > 0);
-    }
-}
-
-// The launch is one cluster.  Levels [0, A.split) run on every block of it;
-// when A.split < A.n - 1 the levels [A.split, A.n) -- a few thousand cells or
-// fewer -- run inside block 0 with block-wide barriers while the other blocks
-// wait at one cluster barrier; otherwise only the coarsest level is left.
-template <typename T>
-__global__ void __launch_bounds__(kTailThreads) k_vtail(const __grid_constant__ TailArgs<T> A) {
-    extern __shared__ double sm[];
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    for (int n = 0; n < A.split; n++) tail_down<true>(A, A.lv[n], A.lv[n + 1], tid, nth);
-    if (A.split < A.n - 1) {
-        if (blockIdx.x == 0) {
-            const int t = threadIdx.x, nt = blockDim.x;
-            for (int n = A.split; n + 1 < A.n; n++) tail_down<false>(A, A.lv[n], A.lv[n + 1], t, nt);
-            tail_coarsest<false>(A, sm, t, nt);
-            for (int n = A.n - 2; n >= A.split; n--) tail_up<false>(A, A.lv[n], A.lv[n + 1], t, nt);
-        }
-        cluster_sync_all();
-    } else {
-        tail_coarsest<true>(A, sm, tid, nth);
-    }
-    for (int n = A.split - 1; n >= 0; n--) tail_up<true>(A, A.lv[n], A.lv[n + 1], tid, nth);
-}
-
-size_t tail_smem(int np, int *mat_in_smem) {
-    const size_t full = sizeof(double) * ((size_t)np + (size_t)np * np);
-    *mat_in_smem = full <= kTailSmemMax ? 1 : 0;
-    return *mat_in_smem ? full : sizeof(double) * (size_t)np;
-}
-
-static cudaLaunchConfig_t tail_cfg(int cl, size_t smem, cudaStream_t s, cudaLaunchAttribute *at) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(kTailThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cfg;
-}
-
-// The largest cluster (16 blocks, else 8) the device can schedule for k_vtail.
-template <typename T>
-cudaError_t tail_grid(size_t smem, int *blocks) {
-    cudaError_t e = cudaFuncSetAttribute(k_vtail<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess && smem > 48 * 1024)
-        e = cudaFuncSetAttribute(k_vtail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    for (int cl = kTailClusterMax; cl >= 8; cl /= 2) {
-        cudaLaunchAttribute at[1];
-        cudaLaunchConfig_t cfg = tail_cfg(cl, smem, nullptr, at);
-        int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, k_vtail<T>, &cfg) == cudaSuccess && nc >= 1) {
-            *blocks = cl;
-            return cudaSuccess;
-        }
-        cudaGetLastError();
-    }
-    return cudaErrorLaunchOutOfResources;
-}
-
-template <typename T>
-cudaError_t launch_vtail(const TailArgs<T> &A, int blocks, size_t smem, cudaStream_t s) {
-    cudaLaunchAttribute at[1];
-    cudaLaunchConfig_t cfg = tail_cfg(blocks, smem, s, at);
-    BB_CHECK_LAUNCH(cudaLaunchKernelEx(&cfg, k_vtail<T>, A));
-    return cudaSuccess;
-}
-
-template cudaError_t tail_grid<double>(size_t, int *);
-template cudaError_t tail_grid<float>(size_t, int *);
-template cudaError_t launch_vtail<double>(const TailArgs<double> &, int, size_t, cudaStream_t);
-template cudaError_t launch_vtail<float>(const TailArgs<float> &, int, size_t, cudaStream_t);
-
 #define BB_INST(T)                                                                                                   \
     template cudaError_t launch_relax<T>(const Lay &, const NbrOff &, int, bool, const T *, T *, const T *, int,     \
                                          cudaStream_t, bool);                                                        \
@@ -2376,8 +2056,6 @@ template cudaError_t launch_vtail<float>(const TailArgs<float> &, int, size_t, c
                                             cudaStream_t);                                                           \
     template cudaError_t launch_restrict<T>(const Lay &, const Lay &, const T *, const T *, T *, T *, cudaStream_t); \
     template cudaError_t launch_prolong<T>(const Lay &, const Lay &, const T *, const T *, T *, cudaStream_t);       \
-    template cudaError_t launch_coarse_solve<T>(const Lay &, const double *, const int *, const int *, const T *,    \
-                                                T *, cudaStream_t);                                                  \
     template cudaError_t launch_maxabs<T>(const Lay &, const T *, double *, double *, cudaStream_t);                \
     template cudaError_t launch_dot<T>(const Lay &, const T *, const T *, double *, double *, cudaStream_t);        \
     template cudaError_t launch_from_caller<T>(const Lay &, const double *, int, T *, cudaStream_t);                 \
