@@ -13,6 +13,7 @@
 // mma.sync with ldmatrix.trans fragments (k_wgrad_mma); everything else is
 // elementwise.
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 
@@ -516,104 +517,140 @@ __global__ void __launch_bounds__(256) k_wgrad(Act x, Act gy, float *__restrict_
     if (db && tap == 13 && blockIdx.z == 0 && threadIdx.x < cout) atomicAdd(&db[threadIdx.x], accb);
 }
 
-// Weight gradient on the tensor cores: for one tap, dW[ci][co] = sum over
-// voxels v of x(v + tap, ci) dy(v, co) is a GEMM with M = ci, N = co and the
-// voxels as K (mma.sync m16n8k16, BF16 products, FP32 accumulation).  A CTA
-// takes one tap, a chunk of voxels and a group of up to kWgTiles output tiles
-// (16 ci x 8 co); per stage it copies kst voxels' channels (a multiple of 128:
-// tap-shifted x with periodic wrap, and dy) as rows of 16-byte chunks into
-// shared memory, its 8 warps take 16 of the voxels at a time as K steps, and
-// ldmatrix.trans turns
-// the channels-last rows into the A (ci x voxel) and B (voxel x co)
-// fragments.  The warps' partial sums meet in shared memory and go to dw with
-// one atomicAdd per output and CTA; the bias gradient (tap 13, tile group 0)
-// is the column sum of dy.  Rows are padded by 16 bytes, so the eight rows an
-// ldmatrix reads fall in distinct banks.
-constexpr int kWgTiles = 8;   // output tiles (16 x 8) per CTA
+// Weight gradient on the tensor cores: dW[tap][ci][co] = sum over voxels v of
+// x(v + tap, ci) dy(v, co) is, per tap, a GEMM with M = ci, N = co and the voxels
+// as K (mma.sync m16n8k16, BF16 products, FP32 accumulation).
+//   * A CTA takes one block of 16 ci x 16 co for all 27 taps, on a tile of 16 (h)
+//     x 16 (w) voxels marching along d: each plane of dy is staged once and each
+//     plane of x (with its halo, periodic wrap) once for the three dz that use it,
+//     instead of once per tap.  Planes are [8-channel group][voxel][16 B] in a
+//     ring of four (x) and two (dy) slots filled with cp.async a plane ahead.
+//   * Nine warps, one per (dz, dy); a K step is one row of 16 voxels.  Its B
+//     fragments (dy) serve the warp's three dx taps, whose A fragments are the
+//     x row shifted by a voxel; ldmatrix.trans turns the channels-last rows into
+//     both (eight consecutive 16-byte rows: no bank conflicts).  Four ldmatrix
+//     feed six MMAs, 24 accumulators per lane.
+//   * The CTA's 27 x 256 sums go to dw with one atomicAdd each; the bias
+//     gradient is an MMA of dy with a matrix of ones.  Voxels beyond the grid and
+//     channels beyond cout are staged as zeros of dy.
+// Measured at 64^3 (the 14 layers of the U-Net): 1.85 ms with one tap per CTA,
+// which read both operands 27 times, 0.30 ms with this kernel.
+constexpr int kWgThreads = 288;
+constexpr int kWgXV = 18 * 18, kWgGV = 16 * 16;         // staged voxels of an x and a dy plane
+constexpr int kWgXB = kWgXV * 32, kWgGB = kWgGV * 32;   // bytes
+constexpr size_t kWgSmem = 4 * kWgXB + 2 * kWgGB;
 
-__device__ __forceinline__ void ldsm_x4_t(unsigned &r0, unsigned &r1, unsigned &r2, unsigned &r3, const void *p) {
+__device__ __forceinline__ void ldsm_x4_t(unsigned &r0, unsigned &r1, unsigned &r2, unsigned &r3, unsigned p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void ldsm_x2_t(unsigned &r0, unsigned &r1, const void *p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(smem_u32(p)));
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(p));
 }
 
-__global__ void __launch_bounds__(256) k_wgrad_mma(Act x, Act gy, float *__restrict__ dw, float *__restrict__ db,
-                                                    int vchunk, int kst) {
-    extern __shared__ __align__(16) unsigned char smw[];
-    const int cin = x.c, cout = gy.c, tap = blockIdx.y;
-    const int xs = cin * 2 + 16, gs = cout * 2 + 16;  // padded row strides (bytes)
-    unsigned char *SX = smw;                                     // [kst][xs]
-    unsigned char *SG = SX + (size_t)kst * xs;                   // [kst][gs]
-    float *red = reinterpret_cast<float *>(SG + (size_t)kst * gs);  // [kWgTiles][128]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int nt = cout >> 3, ntiles = (cin >> 4) * nt;
-    const int tile0 = blockIdx.z * kWgTiles, ntl = min(kWgTiles, ntiles - tile0);
-    const int dz = tap / 9 - 1, dyy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    const int vbeg = blockIdx.x * vchunk, vend = min(vbeg + vchunk, gy.nvox);
-    const bool bias = db && tap == 13 && blockIdx.z == 0;
-    float acc[kWgTiles][4];
+__global__ void __launch_bounds__(kWgThreads) k_wgrad_mma(Act x, Act gy, float *__restrict__ dw,
+                                                           float *__restrict__ db, int tw, int th, int tz, int nz) {
+    extern __shared__ __align__(128) unsigned char smw[];
+    unsigned char *SX = smw, *SG = smw + 4 * kWgXB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cin = x.c, cout = gy.c, nbo = (cout + 15) >> 4;
+    const int ci0 = (blockIdx.y / nbo) * 16, co0 = (blockIdx.y % nbo) * 16;
+    int t = blockIdx.x;
+    const int w0 = (t % tw) * 16;
+    t /= tw;
+    const int h0 = (t % th) * 16;
+    t /= th;
+    const int z0 = (t % tz) * nz, n = t / tz, z1 = min(z0 + nz, x.d);
+    const bf16 *xn = x.p + (long long)n * x.d * x.h * x.w * x.ld + ci0;
+    const bf16 *gn = gy.p + (long long)n * x.d * x.h * x.w * gy.ld + co0;
+    const int xz = x.h * x.w * x.ld, gz = x.h * x.w * gy.ld;
+    // this thread's copies of a plane: chunk e = tid + kWgThreads u is group e & 1 of voxel e >> 1
+    int xo[3], go[2];
 #pragma unroll
-    for (int q = 0; q < kWgTiles; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
-    float accb = 0.f;
-    for (int e = tid; e < kWgTiles * 128; e += 256) red[e] = 0.f;
-    const int cx = cin >> 3, cg = cout >> 3;  // 16-byte chunks per voxel
-    for (int vb = vbeg; vb < vend; vb += kst) {
-        __syncthreads();  // the previous stage is consumed
-        for (int kb = 0; kb < kst; kb += 128) {
-            const int k = kb + (tid & 127), half = tid >> 7, v = vb + k;  // two threads per voxel
-            const bool in = v < vend;
-            long long src = 0;
-            if (in) {
-                int n, d, h, w;
-                decode(gy, v, n, d, h, w);
-                src = (long long)vox(x, n, wrapi(d + dz, x.d), wrapi(h + dyy, x.h), wrapi(w + dx, x.w)) * x.ld;
+    for (int u = 0; u < 3; u++) {
+        const int v = min((tid + kWgThreads * u) >> 1, kWgXV - 1);
+        xo[u] = (wrapn(h0 - 1 + v / 18, x.h) * x.w + wrapn(w0 - 1 + v % 18, x.w)) * x.ld + ((tid + kWgThreads * u) & 1) * 8;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int e = tid + kWgThreads * u, h = h0 + (e >> 5), w = w0 + ((e >> 1) & 15);
+        go[u] = e < 2 * kWgGV && h < x.h && w < x.w && co0 + (e & 1) * 8 < cout ? (h * x.w + w) * gy.ld + (e & 1) * 8 : -1;
+    }
+    auto load_x = [&](int p) {  // plane p of d, in [z0 - 1, z1]
+        const bf16 *src = xn + (long long)wrapn(p, x.d) * xz;
+        unsigned char *dst = SX + (size_t)((p - z0 + 1) & 3) * kWgXB;
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            const int e = tid + kWgThreads * u;
+            if (e < 2 * kWgXV) cpa16(dst + (e & 1) * (kWgXV * 16) + (e >> 1) * 16, src + xo[u]);
+        }
+    };
+    auto load_g = [&](int z) {
+        const bf16 *src = gn + (long long)z * gz;
+        unsigned char *dst = SG + (size_t)((z - z0) & 1) * kWgGB;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int e = tid + kWgThreads * u;
+            if (e >= 2 * kWgGV) continue;
+            unsigned char *d = dst + (e & 1) * (kWgGV * 16) + (e >> 1) * 16;
+            if (go[u] >= 0) cpa16(d, src + go[u]);
+            else *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
+        }
+    };
+    load_x(z0 - 1);
+    load_x(z0);
+    load_x(z0 + 1);
+    load_g(z0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float acc[3][2][4] = {}, accb[2][4] = {};
+    const bool bias = db && warp == 4 && ci0 == 0;
+    const int dz = warp / 3, dy = warp % 3;
+    // ldmatrix: lane L gives the row (L & 7) of matrix L >> 3
+    const int mi = lane >> 3, r8 = lane & 7;
+    const unsigned xa = smem_u32(SX) + ((mi & 1) * kWgXV + (mi >> 1) * 8 + r8 + dy * 18) * 16;  // (ci half, voxel half)
+    const unsigned ga = smem_u32(SG) + ((mi >> 1) * kWgGV + (mi & 1) * 8 + r8) * 16;            // (co half, voxel half)
+    for (int z = z0; z < z1; z++) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // plane z + 1 of x and z of dy are there, the slots of z - 2 and z - 1 free
+        if (z + 1 < z1) {
+            load_x(z + 2);
+            load_g(z + 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const unsigned xs = xa + ((z - z0 + dz) & 3) * kWgXB, gs = ga + ((z - z0) & 1) * kWgGB;
+#pragma unroll 4
+        for (int row = 0; row < 16; row++) {
+            unsigned b0, b1, b2, b3;
+            ldsm_x4_t(b0, b1, b2, b3, gs + row * 256);
+            if (bias) {
+                mma16816(accb[0], 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, b0, b1);
+                mma16816(accb[1], 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, b2, b3);
             }
-            const uint4 zero = make_uint4(0, 0, 0, 0);
-            for (int c = half; c < cx; c += 2)
-                *reinterpret_cast<uint4 *>(SX + (size_t)k * xs + c * 16) =
-                    in ? *reinterpret_cast<const uint4 *>(x.p + src + c * 8) : zero;
-            for (int c = half; c < cg; c += 2)
-                *reinterpret_cast<uint4 *>(SG + (size_t)k * gs + c * 16) =
-                    in ? *reinterpret_cast<const uint4 *>(gy.p + (long long)v * gy.ld + c * 8) : zero;
-        }
-        __syncthreads();
-        for (int k0 = warp * 16; k0 < kst; k0 += 128) {  // this warp's K steps: voxels k0 .. k0+15
 #pragma unroll
-            for (int q = 0; q < kWgTiles; q++) {
-                if (q >= ntl) break;
-                const int tile = tile0 + q, mb = (tile / nt) * 16, nb = (tile % nt) * 8;
-                unsigned a0, a1, a2, a3, b0, b1;
-                const int mi = lane >> 3, r = lane & 7;
-                ldsm_x4_t(a0, a1, a2, a3, SX + (size_t)(k0 + r + (mi >= 2 ? 8 : 0)) * xs + (mb + (mi & 1) * 8) * 2);
-                ldsm_x2_t(b0, b1, SG + (size_t)(k0 + r + ((lane >> 3) & 1) * 8) * gs + nb * 2);
-                mma16816(acc[q], a0, a1, a2, a3, b0, b1);
+            for (int dx = 0; dx < 3; dx++) {
+                unsigned a0, a1, a2, a3;
+                ldsm_x4_t(a0, a1, a2, a3, xs + (row * 18 + dx) * 16);
+                mma16816(acc[dx][0], a0, a1, a2, a3, b0, b1);
+                mma16816(acc[dx][1], a0, a1, a2, a3, b2, b3);
             }
         }
-        if (bias && tid < cout) {
-            for (int k = 0; k < kst; k++)
-                accb += __bfloat162float(reinterpret_cast<const bf16 *>(SG + (size_t)k * gs)[tid]);
+    }
+    // D fragment: rows g, g + 8 (ci), columns 2 t4, 2 t4 + 1 of each co half
+    const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int hf = 0; hf < 2; hf++) {
+        const int co = co0 + hf * 8 + 2 * t4;
+        if (co >= cout) continue;
+#pragma unroll
+        for (int dx = 0; dx < 3; dx++) {
+            float *o = dw + ((long long)(dz * 9 + dy * 3 + dx) * cin + ci0 + g) * cout + co;
+            atomicAdd(o, acc[dx][hf][0]);
+            atomicAdd(o + 1, acc[dx][hf][1]);
+            atomicAdd(o + 8LL * cout, acc[dx][hf][2]);
+            atomicAdd(o + 8LL * cout + 1, acc[dx][hf][3]);
+        }
+        if (bias && g == 0) {
+            atomicAdd(db + co, accb[hf][0]);
+            atomicAdd(db + co + 1, accb[hf][1]);
         }
     }
-    // the 8 warps' partial tiles -> shared memory -> dw
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kWgTiles; q++) {
-        if (q >= ntl) break;
-        // D fragment: rows g / g+8, columns 2 t4, 2 t4 + 1 of the 16 x 8 tile
-        atomicAdd(&red[q * 128 + g * 8 + 2 * t4], acc[q][0]);
-        atomicAdd(&red[q * 128 + g * 8 + 2 * t4 + 1], acc[q][1]);
-        atomicAdd(&red[q * 128 + (g + 8) * 8 + 2 * t4], acc[q][2]);
-        atomicAdd(&red[q * 128 + (g + 8) * 8 + 2 * t4 + 1], acc[q][3]);
-    }
-    __syncthreads();
-    for (int e = tid; e < ntl * 128; e += 256) {
-        const int q = e >> 7, m = (e >> 3) & 15, nn = e & 7;
-        const int tile = tile0 + q, ci = (tile / nt) * 16 + m, co = (tile % nt) * 8 + nn;
-        atomicAdd(&dw[((long long)tap * cin + ci) * cout + co], red[e]);
-    }
-    if (bias && tid < cout) atomicAdd(&db[tid], accb);
 }
 
 // ---------------------------------------------------------------------------
@@ -627,74 +664,106 @@ __global__ void k_pack(const float *__restrict__ w, int cin, int cout, bf16 *__r
     }
 }
 
-__global__ void k_relu_bwd(Act dy, Act y) {
-    const long long n = (long long)dy.nvox * dy.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / dy.c), c = (int)(e % dy.c);
-        if (!(__bfloat162float(y.p[(long long)v * y.ld + c]) > 0.f)) dy.p[(long long)v * dy.ld + c] = __float2bfloat16(0.f);
+// The elementwise kernels take V channels per thread: V = 8 (one 16-byte access)
+// on views whose rows are 16-byte aligned, else 1.
+template <int V> struct Ch {
+    bf16 v[V];
+};
+template <int V> __device__ __forceinline__ Ch<V> ldc(const Act &a, int v, int c) {
+    Ch<V> r;
+    const bf16 *p = a.p + (long long)v * a.ld + c;
+    if (V == 8) *reinterpret_cast<uint4 *>(r.v) = *reinterpret_cast<const uint4 *>(p);
+    else r.v[0] = p[0];
+    return r;
+}
+template <int V> __device__ __forceinline__ void stc(const Act &a, int v, int c, const Ch<V> &r) {
+    bf16 *p = a.p + (long long)v * a.ld + c;
+    if (V == 8) *reinterpret_cast<uint4 *>(p) = *reinterpret_cast<const uint4 *>(r.v);
+    else p[0] = r.v[0];
+}
+#define FOR_CHANNELS(a)                                                                                              \
+    const int cg_ = (a).c / V;                                                                                       \
+    const long long n_ = (long long)(a).nvox * cg_;                                                                  \
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n_; e += (long long)gridDim.x * blockDim.x)
+
+template <int V> __global__ void k_relu_bwd(Act dy, Act y) {
+    FOR_CHANNELS(dy) {
+        const int v = (int)(e / cg_), c = V * (int)(e - (long long)v * cg_);
+        const Ch<V> a = ldc<V>(y, v, c);
+        Ch<V> g = ldc<V>(dy, v, c);
+#pragma unroll
+        for (int q = 0; q < V; q++)
+            if (!(__bfloat162float(a.v[q]) > 0.f)) g.v[q] = __float2bfloat16(0.f);
+        stc<V>(dy, v, c, g);
     }
 }
 
 // y (half size) = mean of the 8 children of x
-__global__ void k_pool2(Act x, Act y) {
-    const long long n = (long long)y.nvox * y.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / y.c), c = (int)(e % y.c);
+template <int V> __global__ void k_pool2(Act x, Act y) {
+    FOR_CHANNELS(y) {
+        const int v = (int)(e / cg_), c = V * (int)(e - (long long)v * cg_);
         int nn, d, h, w;
         decode(y, v, nn, d, h, w);
-        float s = 0.f;
-        for (int q = 0; q < 8; q++)
-            s += __bfloat162float(x.p[(long long)vox(x, nn, 2 * d + (q >> 2), 2 * h + ((q >> 1) & 1), 2 * w + (q & 1)) * x.ld + c]);
-        y.p[(long long)v * y.ld + c] = __float2bfloat16(0.125f * s);
+        Ch<V> in[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) in[q] = ldc<V>(x, vox(x, nn, 2 * d + (q >> 2), 2 * h + ((q >> 1) & 1), 2 * w + (q & 1)), c);
+        Ch<V> o;
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) s += __bfloat162float(in[q].v[m]);
+            o.v[m] = __float2bfloat16(0.125f * s);
+        }
+        stc<V>(y, v, c, o);
     }
 }
 // dx (twice the size of dy) = dy(parent) / 8, or dx += that (accumulate: the
 // pooled tensor is also a skip connection whose gradient is already in dx)
-__global__ void k_pool2_bwd(Act dy, Act dx, int accumulate) {
-    const long long n = (long long)dx.nvox * dx.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / dx.c), c = (int)(e % dx.c);
+template <int V> __global__ void k_pool2_bwd(Act dy, Act dx, int accumulate) {
+    FOR_CHANNELS(dx) {
+        const int v = (int)(e / cg_), c = V * (int)(e - (long long)v * cg_);
         int nn, d, h, w;
         decode(dx, v, nn, d, h, w);
-        float g = 0.125f * __bfloat162float(dy.p[(long long)vox(dy, nn, d >> 1, h >> 1, w >> 1) * dy.ld + c]);
-        bf16 *o = dx.p + (long long)v * dx.ld + c;
-        if (accumulate) g += __bfloat162float(*o);
-        *o = __float2bfloat16(g);
+        const Ch<V> p = ldc<V>(dy, vox(dy, nn, d >> 1, h >> 1, w >> 1), c);
+        Ch<V> o;
+        if (accumulate) o = ldc<V>(dx, v, c);
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            float g = 0.125f * __bfloat162float(p.v[m]);
+            if (accumulate) g += __bfloat162float(o.v[m]);
+            o.v[m] = __float2bfloat16(g);
+        }
+        stc<V>(dx, v, c, o);
     }
 }
 // y (twice the size of x) = x(parent)
-__global__ void k_up2(Act x, Act y) {
-    const long long n = (long long)y.nvox * y.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / y.c), c = (int)(e % y.c);
+template <int V> __global__ void k_up2(Act x, Act y) {
+    FOR_CHANNELS(y) {
+        const int v = (int)(e / cg_), c = V * (int)(e - (long long)v * cg_);
         int nn, d, h, w;
         decode(y, v, nn, d, h, w);
-        y.p[(long long)v * y.ld + c] = x.p[(long long)vox(x, nn, d >> 1, h >> 1, w >> 1) * x.ld + c];
-    }
-}
-// the same, 8 channels (16 bytes) per thread, for 16-byte aligned views
-__global__ void k_up2_v8(Act x, Act y) {
-    const int g8 = y.c >> 3;
-    const long long n = (long long)y.nvox * g8;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / g8), c = 8 * (int)(e - (long long)v * g8);
-        int nn, d, h, w;
-        decode(y, v, nn, d, h, w);
-        *reinterpret_cast<uint4 *>(y.p + (long long)v * y.ld + c) =
-            *reinterpret_cast<const uint4 *>(x.p + (long long)vox(x, nn, d >> 1, h >> 1, w >> 1) * x.ld + c);
+        stc<V>(y, v, c, ldc<V>(x, vox(x, nn, d >> 1, h >> 1, w >> 1), c));
     }
 }
 // dx (half the size of dy) = sum of the 8 children of dy
-__global__ void k_up2_bwd(Act dy, Act dx) {
-    const long long n = (long long)dx.nvox * dx.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / dx.c), c = (int)(e % dx.c);
+template <int V> __global__ void k_up2_bwd(Act dy, Act dx) {
+    FOR_CHANNELS(dx) {
+        const int v = (int)(e / cg_), c = V * (int)(e - (long long)v * cg_);
         int nn, d, h, w;
         decode(dx, v, nn, d, h, w);
-        float s = 0.f;
-        for (int q = 0; q < 8; q++)
-            s += __bfloat162float(dy.p[(long long)vox(dy, nn, 2 * d + (q >> 2), 2 * h + ((q >> 1) & 1), 2 * w + (q & 1)) * dy.ld + c]);
-        dx.p[(long long)v * dx.ld + c] = __float2bfloat16(s);
+        Ch<V> in[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) in[q] = ldc<V>(dy, vox(dy, nn, 2 * d + (q >> 2), 2 * h + ((q >> 1) & 1), 2 * w + (q & 1)), c);
+        Ch<V> o;
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) s += __bfloat162float(in[q].v[m]);
+            o.v[m] = __float2bfloat16(s);
+        }
+        stc<V>(dx, v, c, o);
     }
 }
 
@@ -706,55 +775,85 @@ struct Fields {
 
 // pool = 1: the fields are on x's grid.  pool = 2: they are on the grid twice
 // as fine and each voxel gets the mean of its 8 children (FP64 sum).
-__global__ void k_embed(Fields fs, Act x, int pool) {
-    const long long n = (long long)x.nvox * x.c;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(e / x.c), c = (int)(e % x.c);
-        float val = 0.f;
-        if (c < fs.nf) {
-            if (pool == 1) {
-                val = (float)(fs.s[c] * fs.f[c][v]);
-            } else {
-                int nn, d, h, w;
-                decode(x, v, nn, d, h, w);
-                const int D = 2 * x.d, H = 2 * x.h, W = 2 * x.w;
-                const double *f = fs.f[c] + (long long)nn * D * H * W;
-                double sum = 0.0;
+template <int V> __global__ void k_embed(Fields fs, Act x, int pool) {
+    FOR_CHANNELS(x) {
+        const int v = (int)(e / cg_), c0 = V * (int)(e - (long long)v * cg_);
+        Ch<V> o;
 #pragma unroll
-                for (int q = 0; q < 8; q++)
-                    sum += f[((long long)(2 * d + (q >> 2)) * H + (2 * h + ((q >> 1) & 1))) * W + 2 * w + (q & 1)];
-                val = (float)(fs.s[c] * 0.125 * sum);
+        for (int m = 0; m < V; m++) o.v[m] = __float2bfloat16(0.f);
+        if (c0 < fs.nf) {
+            int nn, d, h, w;
+            if (pool == 2) decode(x, v, nn, d, h, w);
+#pragma unroll
+            for (int m = 0; m < (V < NN_MAX_FIELDS ? V : NN_MAX_FIELDS); m++) {
+                const int c = c0 + m;
+                if (c >= fs.nf) continue;
+                if (pool == 1) {
+                    o.v[m] = __float2bfloat16((float)(fs.s[c] * fs.f[c][v]));
+                } else {
+                    const int D = 2 * x.d, H = 2 * x.h, W = 2 * x.w;
+                    const double *f = fs.f[c] + (long long)nn * D * H * W;
+                    double sum = 0.0;
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                        sum += f[((long long)(2 * d + (q >> 2)) * H + (2 * h + ((q >> 1) & 1))) * W + 2 * w + (q & 1)];
+                    o.v[m] = __float2bfloat16((float)(fs.s[c] * 0.125 * sum));
+                }
             }
         }
-        x.p[(long long)v * x.ld + c] = __float2bfloat16(val);
+        stc<V>(x, v, c0, o);
     }
 }
 
-__global__ void k_head(Act x, const float *__restrict__ w, const float *__restrict__ b, float *__restrict__ out) {
+template <int V> __global__ void k_head(Act x, const float *__restrict__ w, const float *__restrict__ b, float *__restrict__ out) {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < x.nvox; v += gridDim.x * blockDim.x) {
         float s = b[0];
-        for (int c = 0; c < x.c; c++) s = fmaf(__bfloat162float(x.p[(long long)v * x.ld + c]), w[c], s);
+        for (int c = 0; c < x.c; c += V) {
+            const Ch<V> a = ldc<V>(x, v, c);
+#pragma unroll
+            for (int m = 0; m < V; m++) s = fmaf(__bfloat162float(a.v[m]), w[c + m], s);
+        }
         out[v] = s;
     }
 }
 
-__global__ void k_head_bwd(Act x, const float *__restrict__ w, const float *__restrict__ dout, Act dx,
-                           float *__restrict__ dw, float *__restrict__ db) {
-    __shared__ float sw[128], sb;
-    if (threadIdx.x < 128) sw[threadIdx.x] = 0.f;
-    if (threadIdx.x == 0) sb = 0.f;
-    __syncthreads();
+// one group of V channels per blockIdx.y: the sums stay in registers until the
+// grid-stride loop ends, then go over the warp and the block
+template <int V>
+__global__ void __launch_bounds__(256) k_head_bwd(Act x, const float *__restrict__ w, const float *__restrict__ dout,
+                                                   Act dx, float *__restrict__ dw, float *__restrict__ db) {
+    __shared__ float sh[8][V + 1];
+    const int c = blockIdx.y * V, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float acc[V + 1], wc[V];
+#pragma unroll
+    for (int m = 0; m <= V; m++) acc[m] = 0.f;
+#pragma unroll
+    for (int m = 0; m < V; m++) wc[m] = w[c + m];
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < x.nvox; v += gridDim.x * blockDim.x) {
         const float g = dout[v];
-        for (int c = 0; c < x.c; c++) {
-            dx.p[(long long)v * dx.ld + c] = __float2bfloat16(g * w[c]);
-            atomicAdd(&sw[c], g * __bfloat162float(x.p[(long long)v * x.ld + c]));
+        const Ch<V> a = ldc<V>(x, v, c);
+        Ch<V> o;
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            o.v[m] = __float2bfloat16(g * wc[m]);
+            acc[m] += g * __bfloat162float(a.v[m]);
         }
-        atomicAdd(&sb, g);
+        acc[V] += g;
+        stc<V>(dx, v, c, o);
+    }
+#pragma unroll
+    for (int m = 0; m <= V; m++) {
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) acc[m] += __shfl_down_sync(0xffffffffu, acc[m], s);
+        if (lane == 0) sh[warp][m] = acc[m];
     }
     __syncthreads();
-    if (threadIdx.x < x.c) atomicAdd(&dw[threadIdx.x], sw[threadIdx.x]);
-    if (threadIdx.x == 0) atomicAdd(db, sb);
+    if (threadIdx.x <= V) {
+        float s = 0.f;
+        for (int q = 0; q < 8; q++) s += sh[q][threadIdx.x];
+        if (threadIdx.x < V) atomicAdd(dw + c + threadIdx.x, s);
+        else if (blockIdx.y == 0) atomicAdd(db, s);
+    }
 }
 
 __global__ void k_mse(const float *__restrict__ pred, const double *__restrict__ tgt, double scale, long long n,
@@ -824,6 +923,16 @@ int grid_elems(long long n) {
     return (int)(g < 1 ? 1 : g);
 }
 
+// views the elementwise kernels take eight channels at a time
+bool vec8(const Act &a) { return a.c % 8 == 0 && a.ld % 8 == 0 && !(reinterpret_cast<uintptr_t>(a.p) & 15); }
+#define BB_CHANNELS(eight, view, kern, ...)                                                                          \
+    do {                                                                                                             \
+        if (eight)                                                                                                   \
+            kern<8><<<grid_elems((long long)(view).nvox * (view).c / 8), 256, 0, (cudaStream_t)stream>>>(__VA_ARGS__); \
+        else                                                                                                         \
+            kern<1><<<grid_elems((long long)(view).nvox * (view).c), 256, 0, (cudaStream_t)stream>>>(__VA_ARGS__);   \
+    } while (0)
+
 }  // namespace
 
 // ===========================================================================
@@ -855,24 +964,21 @@ int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void
     // tensor cores: channel counts in whole tiles and 16-byte aligned channel rows
     if (!no_mma && ax.c % 16 == 0 && ag.c % 8 == 0 && ax.ld % 8 == 0 && ag.ld % 8 == 0 &&
         !(reinterpret_cast<uintptr_t>(ax.p) & 15) && !(reinterpret_cast<uintptr_t>(ag.p) & 15)) {
-        const int ntiles = (ax.c / 16) * (ag.c / 8), groups = (ntiles + kWgTiles - 1) / kWgTiles;
-        // voxels per stage: 128 x (1..4), up to ~64 KB of staged rows
-        const size_t row = (size_t)(ax.c * 2 + 16 + ag.c * 2 + 16);
-        int kst = 128;
-        while (kst < 512 && (size_t)(2 * kst) * row <= 64 * 1024) kst *= 2;
-        const size_t smem = (size_t)kst * row + sizeof(float) * kWgTiles * 128;
-        static int attr_set = 0;
-        if (smem > 48 * 1024 && !attr_set) {
-            if (cudaFuncSetAttribute(k_wgrad_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(k_wgrad_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem) != cudaSuccess)
                 return BBMG_CUDA;
-            attr_set = 1;
+            attr = true;
         }
-        // about eight CTAs per SM in all: voxel chunks of whole stages
-        int nchunk = (148 * 8 + 27 * groups - 1) / (27 * groups);
-        int vchunk = (ag.nvox + nchunk - 1) / nchunk;
-        vchunk = (vchunk + kst - 1) / kst * kst;
-        nchunk = (ag.nvox + vchunk - 1) / vchunk;
-        k_wgrad_mma<<<dim3(nchunk, 27, groups), 256, smem, (cudaStream_t)stream>>>(ax, ag, dw, db, vchunk, kst);
+        const int tw = (ax.w + 15) / 16, th = (ax.h + 15) / 16, blocks = (ax.c / 16) * ((ag.c + 15) / 16);
+        const long long cols = (long long)tw * th * ax.n;
+        if (blocks > 65535 || cols * ax.d >= (1LL << 31)) return BBMG_BAD_ARGS;
+        // planes per CTA: a CTA ends with 27 x 256 atomic additions, so as many
+        // planes as leave two CTAs per SM
+        int nz = ax.d;
+        while (nz > 1 && cols * blocks * ((ax.d + nz - 1) / nz) < 2 * 148) nz = (nz + 1) / 2;
+        const int tz = (ax.d + nz - 1) / nz;
+        k_wgrad_mma<<<dim3((unsigned)(cols * tz), blocks), kWgThreads, kWgSmem, (cudaStream_t)stream>>>(ax, ag, dw, db, tw, th, tz, nz);
         return done(cudaGetLastError());
     }
     const int chunks = 148 * 4 / 27 + 1;
@@ -903,8 +1009,8 @@ int nn_pack_weights(const float *w, int cin, int cout, void *wt, void *wd, void 
 
 int nn_relu_bwd(const nn_act *dy, const nn_act *y, void *stream) {
     if (bad_act(dy) || bad_act(y) || dy->c != y->c) return BBMG_BAD_ARGS;
-    const Act a = act_of(dy);
-    k_relu_bwd<<<grid_elems((long long)a.nvox * a.c), 256, 0, (cudaStream_t)stream>>>(a, act_of(y));
+    const Act a = act_of(dy), b = act_of(y);
+    BB_CHANNELS(vec8(a) && vec8(b), a, k_relu_bwd, a, b);
     return done(cudaGetLastError());
 }
 
@@ -915,31 +1021,26 @@ static bool halves(const nn_act *big, const nn_act *small) {
 
 int nn_pool2(const nn_act *x, const nn_act *y, void *stream) {
     if (bad_act(x) || bad_act(y) || !halves(x, y)) return BBMG_BAD_ARGS;
-    const Act b = act_of(y);
-    k_pool2<<<grid_elems((long long)b.nvox * b.c), 256, 0, (cudaStream_t)stream>>>(act_of(x), b);
+    const Act a = act_of(x), b = act_of(y);
+    BB_CHANNELS(vec8(a) && vec8(b), b, k_pool2, a, b);
     return done(cudaGetLastError());
 }
 int nn_pool2_bwd(const nn_act *dy, const nn_act *dx, int accumulate, void *stream) {
     if (bad_act(dy) || bad_act(dx) || !halves(dx, dy)) return BBMG_BAD_ARGS;
-    const Act b = act_of(dx);
-    k_pool2_bwd<<<grid_elems((long long)b.nvox * b.c), 256, 0, (cudaStream_t)stream>>>(act_of(dy), b, accumulate);
+    const Act a = act_of(dy), b = act_of(dx);
+    BB_CHANNELS(vec8(a) && vec8(b), b, k_pool2_bwd, a, b, accumulate);
     return done(cudaGetLastError());
 }
 int nn_up2(const nn_act *x, const nn_act *y, void *stream) {
     if (bad_act(x) || bad_act(y) || !halves(y, x)) return BBMG_BAD_ARGS;
     const Act a = act_of(x), b = act_of(y);
-    const bool v8 = b.c % 8 == 0 && a.ld % 8 == 0 && b.ld % 8 == 0 && !(reinterpret_cast<uintptr_t>(a.p) & 15) &&
-                    !(reinterpret_cast<uintptr_t>(b.p) & 15);
-    if (v8)
-        k_up2_v8<<<grid_elems((long long)b.nvox * (b.c >> 3)), 256, 0, (cudaStream_t)stream>>>(a, b);
-    else
-        k_up2<<<grid_elems((long long)b.nvox * b.c), 256, 0, (cudaStream_t)stream>>>(a, b);
+    BB_CHANNELS(vec8(a) && vec8(b), b, k_up2, a, b);
     return done(cudaGetLastError());
 }
 int nn_up2_bwd(const nn_act *dy, const nn_act *dx, void *stream) {
     if (bad_act(dy) || bad_act(dx) || !halves(dy, dx)) return BBMG_BAD_ARGS;
-    const Act b = act_of(dx);
-    k_up2_bwd<<<grid_elems((long long)b.nvox * b.c), 256, 0, (cudaStream_t)stream>>>(act_of(dy), b);
+    const Act a = act_of(dy), b = act_of(dx);
+    BB_CHANNELS(vec8(a) && vec8(b), b, k_up2_bwd, a, b);
     return done(cudaGetLastError());
 }
 
@@ -954,22 +1055,27 @@ int nn_embed(int nf, const double *const *fields, const double *scales, int pool
         fs.s[i] = scales[i];
     }
     const Act a = act_of(x);
-    k_embed<<<grid_elems((long long)a.nvox * a.c), 256, 0, (cudaStream_t)stream>>>(fs, a, pool);
+    BB_CHANNELS(vec8(a), a, k_embed, fs, a, pool);
     return done(cudaGetLastError());
 }
 
 int nn_head(const nn_act *x, const float *w, const float *b, float *out, void *stream) {
     if (bad_act(x) || !w || !b || !out) return BBMG_BAD_ARGS;
     const Act a = act_of(x);
-    k_head<<<grid_elems(a.nvox), 256, 0, (cudaStream_t)stream>>>(a, w, b, out);
+    if (vec8(a)) k_head<8><<<grid_elems(a.nvox), 256, 0, (cudaStream_t)stream>>>(a, w, b, out);
+    else k_head<1><<<grid_elems(a.nvox), 256, 0, (cudaStream_t)stream>>>(a, w, b, out);
     return done(cudaGetLastError());
 }
 
 int nn_head_bwd(const nn_act *x, const float *w, const float *dout, const nn_act *dx, float *dw, float *db,
                 void *stream) {
     if (bad_act(x) || bad_act(dx) || !w || !dout || !dw || !db || x->c > 128 || dx->c != x->c) return BBMG_BAD_ARGS;
-    const Act a = act_of(x);
-    k_head_bwd<<<grid_elems(a.nvox), 256, 0, (cudaStream_t)stream>>>(a, w, dout, act_of(dx), dw, db);
+    const Act a = act_of(x), d = act_of(dx);
+    const unsigned gx = (unsigned)std::min(grid_elems(a.nvox), 148 * 4);
+    if (vec8(a) && vec8(d))
+        k_head_bwd<8><<<dim3(gx, a.c / 8), 256, 0, (cudaStream_t)stream>>>(a, w, dout, d, dw, db);
+    else
+        k_head_bwd<1><<<dim3(gx, a.c), 256, 0, (cudaStream_t)stream>>>(a, w, dout, d, dw, db);
     return done(cudaGetLastError());
 }
 

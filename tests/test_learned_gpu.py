@@ -475,3 +475,24 @@ def test_convolution_tile_edges(L, cin, cout, shape):
     assert L.nn_conv3(C.byref(act(xg, shape)), P(wt), P(bg), C.byref(act(yg, shape)), 1, None) == 0
     assert L.nn_tc_error() == 0
     close_bf16(from_cl(yg, shape), torch.relu(U.conv3(x, wt_, b.double())))
+
+
+@pytest.mark.parametrize("cin,cout,shape", [
+    # one voxel, sizes under and just over a tile of 16 x 16 voxels, an odd plane count, two batches, a half
+    # block of output channels
+    (16, 16, (1, 1, 1, 1)), (32, 48, (1, 5, 17, 18)), (48, 32, (2, 3, 16, 33)), (16, 24, (1, 2, 15, 16)),
+    (128, 128, (1, 2, 2, 2))])
+def test_weight_gradient_tile_edges(L, cin, cout, shape):
+    """Weight and bias gradients on grids that are not whole tiles, against the oracle."""
+    rng = np.random.default_rng(13 * cin + cout)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    dy = bf(rng.standard_normal((n, cout, d, h, w)))
+    dw = torch.zeros(27 * cin * cout, dtype=torch.float32, device="cuda")
+    db = torch.zeros(cout, dtype=torch.float32, device="cuda")
+    xg, dyg = to_cl(x), to_cl(dy)
+    assert L.nn_conv3_wgrad(C.byref(act(xg, shape)), C.byref(act(dyg, shape)), P(dw), P(db), None) == 0
+    rw, rb = U.conv3_wgrad(x, dy)
+    tol = 1e-4 * float(np.sqrt(n * d * h * w))  # FP32 sums of V unit products
+    np.testing.assert_allclose(dw.cpu().double().numpy().reshape(27, cin, cout), rw.numpy(), rtol=0, atol=tol)
+    np.testing.assert_allclose(db.cpu().double().numpy(), rb.numpy(), rtol=0, atol=tol)
