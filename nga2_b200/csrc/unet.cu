@@ -411,10 +411,10 @@ int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y
     ZmGeo g;
     g.tw = (x.w + 7) / 8;
     g.th = (x.h + 15) / 16;
-    // output planes per tile: as many as 256 TMEM columns hold (two CTAs share
+    // output planes per tile: as many as 128 TMEM columns hold (four CTAs share
     // an SM's 512), fewer where that would leave SMs idle
     const long long cols = (long long)g.tw * g.th * x.n;
-    g.dz = min(x.d, max(1, 256 / N));
+    g.dz = min(x.d, max(1, 128 / N));
     while (g.dz > 1 && cols * ((x.d + g.dz - 1) / g.dz) < 2 * 148) g.dz = (g.dz + 1) / 2;
     g.tz = (x.d + g.dz - 1) / g.dz;
     for (g.cols = 32; g.cols < g.dz * N;) g.cols *= 2;
