@@ -7,16 +7,21 @@
 // residual, restriction, prolongation) reads v from the block's own shared
 // memory, writes each new value there and, at a slab face or a periodic face,
 // straight into the neighbour's copy (distributed shared memory); the cluster's
-// hardware barrier ends the pass.  The operator planes stay in global memory
-// (L2): they do not depend on the pass before, so a pass loads its first
-// point's coefficients into registers between arriving at a barrier and
+// hardware barrier ends the pass.  The operator does not depend on the pass
+// before: the coefficients of the coarser levels are staged in shared memory
+// before the wait for the predecessor, as many levels as fit, and those of the
+// others are loaded from L2 into registers between arriving at a barrier and
 // waiting for it.  Levels of at most kTailSingle cells, and always the coarsest,
 // run inside block 0 with block-wide barriers while the others wait.
 //
-// What bounds it: a pass is a chain of latencies (barrier, 27 shared-memory
-// loads, a sum in the reference's order, a division), no longer a kernel launch
-// or an L2 round trip for v.  A cluster is scheduled as a unit, so no block can
-// wait on one that is not running, and no barrier outlives its kernel.
+// What bounds it: a pass is a chain of latencies (barrier 0.4e3 cycles, shared
+// memory loads, a sum in the reference's order, a division) of a few warps, no
+// longer a kernel launch or an L2 round trip for v; FP64 levels of 16^3 and 32^3
+// wait for their coefficients from L2.  With the levels below 8^3 fused and the
+// others one launch per colour, a 32^3 mixed solve took 3.13 ms and a 64^3 FP64
+// one 4.19; fused from 32^3 they take 1.62 and 2.75 ms.  A cluster is scheduled
+// as a unit, so no block can wait on one that is not running, and no barrier
+// outlives its kernel.
 //
 // Arithmetic and term order are those of the single-pass kernels (solve.cu):
 // FP64 results are the oracle's bits.

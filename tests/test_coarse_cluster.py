@@ -1,0 +1,66 @@
+"""The coarse levels that run in one cluster launch: slab splits and edges.
+
+Whole FP64 cycles and solves equal the oracle bit for bit where the levels are
+dealt out unevenly over the blocks (more planes than blocks, a last block with
+fewer, fewer planes than blocks), with odd periodic sizes and with an odd number
+of sweeps; coarsest systems below, at and above the sizes its solve is written
+for are checked through the direct solve."""
+import numpy as np
+import pytest
+
+from nga2_b200 import problems as P
+
+pytestmark = pytest.mark.gpu
+
+SLABS = [((40, 24, 36), (True, False, True)),   # three planes a block, the last blocks without any
+         ((24, 20, 17), (False, True, False)),  # two planes a block, the last with one
+         ((64, 40, 12), (True, True, True)),    # fewer planes than blocks
+         ((21, 18, 35), (True, False, True)),   # odd periodic sizes
+         ((36, 32, 32), (True, True, True))]    # the largest first level
+
+
+def pair(dims, per, seed=3, **kw):
+    from nga2_b200.bbmg import BBMG, BBOX, FP64
+    from oracle.oracle import OracleBBMG
+    stc, opr = P.random_operator(*dims, per, seed=seed)
+    o = OracleBBMG(*dims, *per, method=BBOX, **kw)
+    o.setup(stc, opr)
+    g = BBMG(*dims, *per, method=BBOX, precision=FP64, **kw)
+    g.setup(stc, opr)
+    return o, g
+
+
+@pytest.mark.parametrize("dims,per", SLABS)
+def test_slab_splits_bitexact(dims, per):
+    o, g = pair(dims, per, maxit=3, rcvg=0.0)
+    b = np.random.default_rng(5).standard_normal(dims[::-1])
+    b -= b.mean()
+    xo, ito, ro = o.solve(b)
+    xg, itg, rg, _ = g.solve(b)
+    assert ito == itg and ro == rg
+    assert np.array_equal(xo, xg)
+
+
+@pytest.mark.parametrize("pre,post", [(1, 2), (3, 1), (0, 2)])
+def test_sweep_counts_bitexact(pre, post):
+    o, g = pair((20, 12, 18), (True, False, True), maxit=2, rcvg=0.0, relax_pre=pre, relax_post=post)
+    b = np.random.default_rng(6).standard_normal((18, 12, 20))
+    b -= b.mean()
+    xo, _, ro = o.solve(b)
+    xg, _, rg, _ = g.solve(b)
+    assert ro == rg and np.array_equal(xo, xg)
+
+
+@pytest.mark.parametrize("dims", [(2, 3, 1), (4, 4, 2), (4, 4, 4), (5, 5, 4), (8, 8, 2), (8, 6, 3), (8, 6, 6)])
+def test_coarsest_solve_sizes(dims):
+    """6 to 288 unknowns: registers of one and two lanes' worth, factors on and off chip."""
+    o, g = pair(dims, (False, False, False), seed=9, ncell_coarsest=300)
+    n = g.nlvl
+    nx, ny, nz = g.level_dims(n)
+    f = np.zeros((nz + 2, ny + 2, nx + 2))
+    f[1:-1, 1:-1, 1:-1] = np.random.default_rng(8).standard_normal((nz, ny, nx))
+    o.put(n, "f", f)
+    g.put(n, "f", f)
+    o.direct_solve()
+    g.step("direct", n)
+    assert np.array_equal(g.get(n, "v"), o.get(n, "v"))
