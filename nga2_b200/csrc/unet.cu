@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(128) k_conv3(Act x, const bf16 *__restrict__ w
 //   * A planes sit in a ring of kZmA slots filled with cp.async kZmA - 1
 //     stages ahead; one thread issues a stage's MMAs and commits them to the
 //     slot's mbarrier, which gates its refill.  The weights of a chunk have NB
-//     buffers; with one, the next chunk's load waits for the MMAs before it.
+//     buffers; with one, the next chunk's load waits for the MMAs before it.  A
+//     tile of one output plane has the weights of each stage's dz in its slot.
 //   * The epilogue reads the four warps' 32 TMEM lanes, adds the bias, applies
 //     the ReLU and stores BF16.
 // Measured at 128^3 (the whole forward pass of the U-Net with its guess assembly):
@@ -201,7 +202,7 @@ struct ZmGeo {
     int tw, th, tz;  // tiles along w, h, d
     int dz;          // output planes per tile
     int cols;        // TMEM columns
-    int nb;          // weight buffers
+    int nb;          // weight buffers; 0: with one output plane per tile, weights in the plane's stage
 };
 
 __device__ __forceinline__ int wrapn(int i, int n) {
@@ -213,6 +214,7 @@ template <int N>
 __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict__ wt, const float *__restrict__ bias,
                                                    Act y, int relu, ZmGeo geo, int *err) {
     constexpr int kB = 27 * N * 32;  // bytes of a chunk's weights
+    constexpr int kB3 = kB / 3;      // of one dz of it
     extern __shared__ __align__(128) unsigned char smtc[];
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(smtc);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smtc + 16);  // kZmA barriers
@@ -258,20 +260,32 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
     };
     // weights of chunk c: [dy, dx][group][dz = +1, 0, -1][cout][16 B]
     auto load_b = [&](int c) {
-        unsigned char *Bs = B + (size_t)(c % geo.nb) * kB;
+        unsigned char *Bs = B + (size_t)(c % geo.nb) * kB;  // nb >= 1
         for (int e = tid; e < 54 * N; e += 128) {
             const int g = e & 1, o = (e >> 1) % N, tap = (e >> 1) / N;  // tap = 9 dz + 3 dy + dx
             const int dzi = tap / 9, t9 = tap - 9 * dzi;
             cpa16(Bs + (((t9 * 2 + g) * 3 + 2 - dzi) * N + o) * 16, wt + ((long long)tap * N + o) * cin + c * 16 + g * 8);
         }
     };
+    // one output plane: stage st (input plane st % 3 of chunk st / 3) has only the
+    // taps of one dz, and they come with it: [dy, dx][group][cout][16 B]
+    const bool third = geo.nb == 0;
+    auto load_b3 = [&](int st) {
+        const int c = st / 3, r = st - 3 * c;
+        unsigned char *Bs = B + (size_t)(st % kZmA) * kB3;
+        for (int e = tid; e < 18 * N; e += 128) {
+            const int g = e & 1, o = (e >> 1) % N, t9 = (e >> 1) / N;
+            cpa16(Bs + ((t9 * 2 + g) * N + o) * 16, wt + ((long long)(9 * r + t9) * N + o) * cin + c * 16 + g * 8);
+        }
+    };
     auto commit_group = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-    load_b(0);
+    if (!third) load_b(0);
 #pragma unroll 1
     for (int p = 0; p < kZmA - 1; p++) {
         if (p < nst) {
-            if (p && p % npl == 0 && geo.nb > 1) load_b(p / npl);
+            if (third) load_b3(p);
+            else if (p && p % npl == 0 && geo.nb > 1) load_b(p / npl);
             load_a(p);
         }
         commit_group();
@@ -307,7 +321,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned as = smem_u32(A + (size_t)(st % kZmA) * kZmPlane), bs = smem_u32(B + (size_t)(c % geo.nb) * kB);
+            const unsigned as = smem_u32(A + (size_t)(st % kZmA) * kZmPlane), bs = smem_u32(third ? B + (size_t)(st % kZmA) * kB3 : B + (size_t)(c % geo.nb) * kB);
             // output planes lo .. hi (tile-local) of input plane r - 1
             const int lo = max(0, r - 2), hi = min(nq - 1, r), b0 = lo - (r - 2);
             const int nblk = hi - lo + 1, per = 3 * N <= 256 ? nblk : 1;
@@ -315,6 +329,10 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
 #pragma unroll 1
             for (int t9 = 0; t9 < 9; t9++) {
                 const uint64_t ad = umma_desc(as + ((t9 / 3) * 10 + t9 % 3) * 16, kZmVox * 16, 160);
+                if (third) {
+                    umma_bf16(tmem, ad, umma_desc(bs + t9 * 2 * N * 16, N * 16, 128), umma_idesc_bf16(N));
+                    continue;
+                }
                 for (int b = 0; b < nblk; b += per)
                     umma_bf16(tmem + (lo + b) * N, ad, umma_desc(bs + (t9 * 6 + b0 + b) * N * 16, 3 * N * 16, 128), idesc);
             }
@@ -330,7 +348,8 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
                     break;
                 }
             }
-            if (nx % npl == 0 && geo.nb > 1) load_b(nx / npl);
+            if (third) load_b3(nx);
+            else if (nx % npl == 0 && geo.nb > 1) load_b(nx / npl);
             load_a(nx);
         }
         commit_group();
@@ -418,13 +437,19 @@ int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y
     while (g.dz > 1 && cols * ((x.d + g.dz - 1) / g.dz) < 2 * 148) g.dz = (g.dz + 1) / 2;
     g.tz = (x.d + g.dz - 1) / g.dz;
     for (g.cols = 32; g.cols < g.dz * N;) g.cols *= 2;
-    // two weight buffers where two CTAs per SM still fit with them, or where
-    // only one fits anyway
+    // One plane per tile (the deep levels: few tiles, long K): each stage brings
+    // the weights of its own dz, so that no load waits for a whole chunk's MMAs.
+    // Average per layer of the network's 64- and 128-channel convolutions on 64^3:
+    // 36 and 65 us with one weight buffer per chunk, 33 and 56 us so.
+    // Otherwise two weight buffers where two CTAs per SM still fit with them, or
+    // where only one fits anyway.
     const bool two = kFixed + 2 * kB <= kTwoPerSm || (kFixed + kB > kTwoPerSm && kFixed + 2 * kB <= kMost);
-    g.nb = x.c > 16 && two ? 2 : 1;
+    constexpr bool thirds = kFixed + kZmA * (kB / 3) <= kMost;
+    g.nb = g.dz == 1 && thirds ? 0 : (x.c > 16 && two ? 2 : 1);
     const long long grid = cols * g.tz;
     if (grid >= (1LL << 31)) return BBMG_BAD_ARGS;
-    k_conv3_zm<N><<<(unsigned)grid, 128, kFixed + g.nb * kB, s>>>(x, wt, bias, y, relu, g, err);
+    const int smem = kFixed + (g.nb ? g.nb * kB : kZmA * (kB / 3));
+    k_conv3_zm<N><<<(unsigned)grid, 128, smem, s>>>(x, wt, bias, y, relu, g, err);
     return done(cudaGetLastError());
 }
 
