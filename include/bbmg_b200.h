@@ -207,7 +207,12 @@ const char *bbmg_last_error(const bbmg_handle *h);
  * of f2c and oprc2f is read by nothing in the setup or the solve; on levels
  * with even sizes the setup leaves it unfilled, and bbmg_debug_get fills it
  * (zero in non-periodic directions, the periodic image otherwise, as the
- * reference holds it) on the handle's stream before the copy out. */
+ * reference holds it) on the handle's stream before the copy out.
+ * bbmg_debug_step runs each pass as a launch of its own and leaves v, f and r of
+ * every level in place.  bbmg_solve and bbmg_profile_step run the coarse levels
+ * inside one launch that keeps vectors on chip: the first of those levels gets
+ * its V (not R) written, and the V, F and R of the levels below it still hold
+ * what the last step or put left there. */
 long long bbmg_debug_get(bbmg_handle *h, int level, int which, int prec, double *out);
 long long bbmg_debug_put(bbmg_handle *h, int level, int which, int prec, const double *in);
 int bbmg_debug_step(bbmg_handle *h, int step, int level, int arg, int prec);

@@ -64,3 +64,27 @@ def test_coarsest_solve_sizes(dims):
     o.direct_solve()
     g.step("direct", n)
     assert np.array_equal(g.get(n, "v"), o.get(n, "v"))
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("dims,per", SLABS)
+def test_cycle_leaves_the_vectors_of_every_level(monkeypatch, dims, per, prec):
+    """v, f and r of all levels after a cycle, overlap included, equal those of one launch per pass."""
+    from nga2_b200.bbmg import BBMG, FP64, MIXED, PCG_BBOX
+    stc, opr = P.random_operator(*dims, per, seed=3)
+    rng = np.random.default_rng(4)
+    f = rng.standard_normal(tuple(n + 2 for n in dims[::-1]))
+    got = []
+    for cells in (None, "0"):
+        if cells:
+            monkeypatch.setenv("BBMG_TAIL_CELLS", cells)
+        h = BBMG(*dims, *per, method=PCG_BBOX, precision=MIXED if prec else FP64)
+        h.setup(stc, opr)
+        h.put(1, "v", np.zeros_like(f), prec)
+        h.put(1, "f", f, prec)
+        h.step("cycle", 1, 0, prec)
+        got.append([{w: h.get(n, w, prec) for w in ("v", "f", "r")} for n in range(1, h.nlvl + 1)])
+        h.close()
+    for n, (a, b) in enumerate(zip(*got)):
+        for w in ("v", "f", "r"):
+            assert np.array_equal(a[w], b[w]), (n + 1, w)
