@@ -34,8 +34,14 @@ typedef struct {
 /* y = act(conv3x3x3(x, w) + bias); act = ReLU when relu != 0.  wt is the
  * forward packing of nn_pack_weights.  Tensor cores with FP32 accumulation:
  * tcgen05.mma with TMEM accumulators for cout 16, 32, 48, 64, 96, 128 and 192
- * on 16-byte aligned views (any grid), mma.sync otherwise. */
+ * on 16-byte aligned views and weights (any grid), mma.sync otherwise. */
 int nn_conv3(const nn_act *x, const void *wt, const float *bias, const nn_act *y, int relu, void *stream);
+
+/* How nn_conv3(x, wt, ..., y) or nn_conv3_dgrad(x, wt, y) would run: *tcgen05 = 1
+ * on tcgen05.mma, 0 on mma.sync; on tcgen05 the output planes a tile holds and
+ * its weight buffers (0: the weights come with each input plane).  Looks at the
+ * sizes and addresses only and launches nothing. */
+int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers);
 
 /* BBMG_CUDA if a tcgen05 convolution's completion wait ran out since the last
  * call (the flag is then cleared), else 0.  Synchronises the device. */

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "../../include/bbmg_b200.h"
 #include "../../include/bbmg_learned.h"
@@ -405,28 +406,26 @@ int *tc_err_flag() {
     return flag;
 }
 
-// the tcgen05 path: 16-byte aligned channel rows and an output width the
-// kernel is instantiated for
-bool tc_eligible(const Act &x, const Act &y) {
+// the tcgen05 path: 16-byte aligned channel rows and weights (all three are
+// copied 16 bytes at a time) and an output width the kernel is instantiated for
+bool tc_eligible(const Act &x, const bf16 *wt, const Act &y) {
     static const bool off = getenv("BBMG_NO_TCGEN05") != nullptr;
     if (off || x.c % 16) return false;
     if (y.c != 16 && y.c != 32 && y.c != 48 && y.c != 64 && y.c != 96 && y.c != 128 && y.c != 192) return false;
-    return !(x.ld % 8 || y.ld % 8 || (reinterpret_cast<uintptr_t>(x.p) & 15) || (reinterpret_cast<uintptr_t>(y.p) & 15));
+    const auto off16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+    return !(x.ld % 8 || y.ld % 8 || off16(x.p) || off16(wt) || off16(y.p));
 }
 
-template <int N>
-int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
-    constexpr int kFixed = 128 + kZmA * kZmPlane, kB = 27 * N * 32;
-    constexpr int kTwoPerSm = 112 * 1024, kMost = 226 * 1024;
+template <int N> struct ZmCfg {
+    static constexpr int kFixed = 128 + kZmA * kZmPlane, kB = 27 * N * 32;
+    static constexpr int kTwoPerSm = 112 * 1024, kMost = 226 * 1024;
     static_assert(kFixed + kB <= kMost, "one weight buffer has to fit");
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv3_zm<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess)
-            return BBMG_CUDA;
-        attr = true;
-    }
-    int *err = tc_err_flag();
-    if (!err) return BBMG_NO_MEMORY;
+    static constexpr bool kThirds = kFixed + kZmA * (kB / 3) <= kMost;
+};
+
+template <int N>
+ZmGeo conv_geo(const Act &x) {
+    using Cfg = ZmCfg<N>;
     ZmGeo g;
     g.tw = (x.w + 7) / 8;
     g.th = (x.h + 15) / 16;
@@ -443,29 +442,50 @@ int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y
     // 36 and 65 us with one weight buffer per chunk, 33 and 56 us so.
     // Otherwise two weight buffers where two CTAs per SM still fit with them, or
     // where only one fits anyway.
-    const bool two = kFixed + 2 * kB <= kTwoPerSm || (kFixed + kB > kTwoPerSm && kFixed + 2 * kB <= kMost);
-    constexpr bool thirds = kFixed + kZmA * (kB / 3) <= kMost;
-    g.nb = g.dz == 1 && thirds ? 0 : (x.c > 16 && two ? 2 : 1);
-    const long long grid = cols * g.tz;
+    constexpr bool two = Cfg::kFixed + 2 * Cfg::kB <= Cfg::kTwoPerSm ||
+                         (Cfg::kFixed + Cfg::kB > Cfg::kTwoPerSm && Cfg::kFixed + 2 * Cfg::kB <= Cfg::kMost);
+    g.nb = g.dz == 1 && Cfg::kThirds ? 0 : (x.c > 16 && two ? 2 : 1);
+    return g;
+}
+
+template <int N>
+int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
+    using Cfg = ZmCfg<N>;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(k_conv3_zm<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kMost) != cudaSuccess)
+            return BBMG_CUDA;
+        attr = true;
+    }
+    int *err = tc_err_flag();
+    if (!err) return BBMG_NO_MEMORY;
+    const ZmGeo g = conv_geo<N>(x);
+    const long long grid = (long long)g.tw * g.th * x.n * g.tz;
     if (grid >= (1LL << 31)) return BBMG_BAD_ARGS;
-    const int smem = kFixed + (g.nb ? g.nb * kB : kZmA * (kB / 3));
+    const int smem = Cfg::kFixed + (g.nb ? g.nb * Cfg::kB : kZmA * (Cfg::kB / 3));
     k_conv3_zm<N><<<(unsigned)grid, 128, smem, s>>>(x, wt, bias, y, relu, g, err);
     return done(cudaGetLastError());
 }
 
+// f(output width as a constant) for the widths of tc_eligible
+template <typename F>
+int with_width(int n, F f) {
+    switch (n) {
+    case 16: return f(std::integral_constant<int, 16>{});
+    case 32: return f(std::integral_constant<int, 32>{});
+    case 48: return f(std::integral_constant<int, 48>{});
+    case 64: return f(std::integral_constant<int, 64>{});
+    case 96: return f(std::integral_constant<int, 96>{});
+    case 128: return f(std::integral_constant<int, 128>{});
+    case 192: return f(std::integral_constant<int, 192>{});
+    }
+    return BBMG_BAD_ARGS;
+}
+
 int launch_conv(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
     const int blocks = (x.nvox + 63) / 64;
-    if (tc_eligible(x, y)) {
-        switch (y.c) {
-        case 16: return launch_conv_tc<16>(x, wt, bias, y, relu, s);
-        case 32: return launch_conv_tc<32>(x, wt, bias, y, relu, s);
-        case 48: return launch_conv_tc<48>(x, wt, bias, y, relu, s);
-        case 64: return launch_conv_tc<64>(x, wt, bias, y, relu, s);
-        case 96: return launch_conv_tc<96>(x, wt, bias, y, relu, s);
-        case 128: return launch_conv_tc<128>(x, wt, bias, y, relu, s);
-        case 192: return launch_conv_tc<192>(x, wt, bias, y, relu, s);
-        }
-    }
+    if (tc_eligible(x, wt, y))
+        return with_width(y.c, [&](auto n) { return launch_conv_tc<decltype(n)::value>(x, wt, bias, y, relu, s); });
     // output widths of the U-Net: 16/32/64/128 forward; the data gradients
     // of the concatenated decoder inputs add 48/96/192
     if (y.c % 8) return BBMG_BAD_ARGS;
@@ -978,6 +998,20 @@ int nn_conv3_dgrad(const nn_act *dy, const void *wd, const nn_act *dx, void *str
         dy->h != dx->h || dy->w != dx->w)
         return BBMG_BAD_ARGS;
     return launch_conv(act_of(dy), (const bf16 *)wd, nullptr, act_of(dx), 0, (cudaStream_t)stream);
+}
+
+int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers) {
+    if (bad_act(x) || bad_act(y) || !wt || !tcgen05 || !planes || !buffers) return BBMG_BAD_ARGS;
+    const Act ax = act_of(x), ay = act_of(y);
+    *tcgen05 = tc_eligible(ax, (const bf16 *)wt, ay);
+    *planes = *buffers = 0;
+    if (!*tcgen05) return BBMG_OK;
+    return with_width(ay.c, [&](auto n) {
+        const ZmGeo g = conv_geo<decltype(n)::value>(ax);
+        *planes = g.dz;
+        *buffers = g.nb;
+        return BBMG_OK;
+    });
 }
 
 int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void *stream) {

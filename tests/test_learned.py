@@ -1,6 +1,7 @@
 """Learned initial guess, host side: the U-Net oracle (checked against direct
 sums and finite differences), the parameter layout shared with the CUDA
 kernels, the C ABI's nn_* exports, and the solve-sequence generator."""
+import ctypes as C
 import os
 import re
 
@@ -179,3 +180,26 @@ def test_turbulence_sequence_projection_and_decay():
         assert rec["opr"].shape == (16, 16, 16, 7)
     urms = (float(sum((x ** 2).mean() for x in seq.u)) / 3) ** 0.5
     assert urms < urms0
+
+
+def test_unaligned_weights_do_not_take_the_16_byte_copies():
+    """The path a convolution takes by its addresses alone (nothing is launched): tcgen05 copies x and the
+    weights 16 bytes at a time, and its epilogue stores y so; anything else goes to mma.sync."""
+    L = NL.lib()
+
+    def path(cin, cout, shape=(1, 5, 16, 8), xo=0, wo=0, yo=0, ld=0):
+        x = NL.Act(0x10000000 + xo, *shape, cin, cin + ld)
+        y = NL.Act(0x20000000 + yo, *shape, cout, cout)
+        tc, planes, buf = C.c_int(-1), C.c_int(-1), C.c_int(-1)
+        assert L.bbmg_debug_conv3(C.byref(x), 0x30000000 + wo, C.byref(y), C.byref(tc), C.byref(planes),
+                                  C.byref(buf)) == 0
+        return tc.value
+
+    for cin, cout in ((16, 16), (192, 64), (128, 128), (64, 192)):
+        assert path(cin, cout) == 1
+        assert path(cin, cout, (1, 1, 1, 1)) == 1
+        for off in (4, 8, 12):
+            assert path(cin, cout, wo=off) == 0, off
+            assert path(cin, cout, xo=off) == 0 and path(cin, cout, yo=off) == 0
+        assert path(cin, cout, ld=8) == 1 and path(cin, cout, ld=2) == 0
+    assert path(16, 80) == 0

@@ -73,6 +73,13 @@ def packed(L, w):
     return wt, wd
 
 
+def tiling(L, x, wt, y):
+    """(tcgen05, output planes per tile, weight buffers) that a convolution would run with."""
+    r = [C.c_int(-1) for _ in range(3)]
+    assert L.bbmg_debug_conv3(C.byref(x), wt, C.byref(y), *map(C.byref, r)) == 0
+    return tuple(v.value for v in r)
+
+
 @pytest.mark.parametrize("cin,cout,relu,shape", [(16, 16, 1, (1, 6, 10, 12)), (48, 32, 0, (2, 4, 4, 8)),
                                                  (192, 64, 1, (1, 4, 6, 4)), (64, 128, 1, (1, 4, 4, 4)),
                                                  (32, 16, 0, (1, 3, 5, 7))])
@@ -496,3 +503,24 @@ def test_weight_gradient_tile_edges(L, cin, cout, shape):
     tol = 1e-4 * float(np.sqrt(n * d * h * w))  # FP32 sums of V unit products
     np.testing.assert_allclose(dw.cpu().double().numpy().reshape(27, cin, cout), rw.numpy(), rtol=0, atol=tol)
     np.testing.assert_allclose(db.cpu().double().numpy(), rb.numpy(), rtol=0, atol=tol)
+
+
+def test_convolution_of_a_packed_slice(L):
+    """Weights that start 4 bytes into a buffer: mma.sync, against the oracle."""
+    cin, cout, shape = 32, 48, (1, 5, 7, 9)
+    rng = np.random.default_rng(17)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    wt_ = bf(rng.standard_normal((27, cin, cout)) / np.sqrt(27 * cin))
+    wt, wd = packed(L, wt_.numpy())
+    buf = torch.zeros(wt.numel() + 2, dtype=torch.bfloat16, device="cuda")
+    part = buf[2:]
+    xg, yg = to_cl(x), torch.empty((n * d * h * w, cout), dtype=torch.bfloat16, device="cuda")
+    assert tiling(L, act(xg, shape), P(part), act(yg, shape))[0] == 0
+    part.copy_(wt)
+    assert L.nn_conv3(C.byref(act(xg, shape)), P(part), None, C.byref(act(yg, shape)), 0, None) == 0
+    close_bf16(from_cl(yg, shape), U.conv3(x, wt_, torch.zeros(cout, dtype=torch.float64)))
+    part.copy_(wd)
+    dxg = torch.empty_like(xg)
+    assert L.nn_conv3_dgrad(C.byref(act(yg, shape)), P(part), C.byref(act(dxg, shape)), None) == 0
+    close_bf16(from_cl(dxg, shape), U.conv3_dgrad(from_cl(yg, shape), wt_))
