@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
                       "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                     : "r"(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(q * N + c0)));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                __nv_bfloat162 o2[8];
+                alignas(16) __nv_bfloat162 o2[8];
 #pragma unroll
                 for (int m = 0; m < 8; m++) {
                     float a = __uint_as_float(v[2 * m]) + (bias ? bias[c0 + 2 * m] : 0.f);
@@ -710,10 +710,11 @@ __global__ void k_pack(const float *__restrict__ w, int cin, int cout, bf16 *__r
 }
 
 // The elementwise kernels take V channels per thread: V = 8 (one 16-byte access)
-// on views whose rows are 16-byte aligned, else 1.
-template <int V> struct Ch {
+// on views whose rows are 16-byte aligned, else 1.  Ch is aligned as its access is.
+template <int V> struct alignas(V == 8 ? 16 : 2) Ch {
     bf16 v[V];
 };
+static_assert(alignof(Ch<8>) == 16 && sizeof(Ch<8>) == 16 && sizeof(Ch<1>) == 2, "accessed as one vector");
 template <int V> __device__ __forceinline__ Ch<V> ldc(const Act &a, int v, int c) {
     Ch<V> r;
     const bf16 *p = a.p + (long long)v * a.ld + c;
