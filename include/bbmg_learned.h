@@ -43,8 +43,9 @@ int nn_conv3(const nn_act *x, const void *wt, const float *bias, const nn_act *y
  * sizes and addresses only and launches nothing. */
 int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers);
 
-/* BBMG_CUDA if a tcgen05 convolution's completion wait ran out since the last
- * call (the flag is then cleared), else 0.  Synchronises the device. */
+/* BBMG_CUDA if a tcgen05 convolution's completion wait ran out on the current
+ * device since the last call (the flag is then cleared), else 0.  Synchronises
+ * the device. */
 int nn_tc_error(void);
 
 /* dx = conv3x3x3 of dy with the mirrored, transposed weights (wd, the

@@ -14,6 +14,7 @@
 // elementwise.
 #include <cuda_bf16.h>
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <type_traits>
@@ -148,9 +149,10 @@ __global__ void __launch_bounds__(128) k_conv3(Act x, const bf16 *__restrict__ w
 // Measured at 128^3 (the whole forward pass of the U-Net with its guess assembly):
 // 3.55 ms with one CTA per 128-voxel row tile that staged an input row for each
 // (dz, dy) and issued 27 MMAs of N = cout per tile, 1.71 ms with this kernel.
-// Every mbarrier wait is bounded: a wait that runs out raises *err (read by
+// Every mbarrier wait is bounded: a wait that runs out raises g_tc_err (read by
 // nn_tc_error), and the CTA then drains its copies, frees its TMEM and returns
 // without writing.
+__device__ int g_tc_err;  // each device's own, there without an allocation: a first call may be captured
 constexpr unsigned kTcSpinLimit = 1u << 22;
 constexpr int kZmA = 4;                     // A slots
 constexpr int kZmVox = 10 * 18;             // voxels of a halo plane
@@ -213,7 +215,7 @@ __device__ __forceinline__ int wrapn(int i, int n) {
 
 template <int N>
 __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict__ wt, const float *__restrict__ bias,
-                                                   Act y, int relu, ZmGeo geo, int *err) {
+                                                   Act y, int relu, ZmGeo geo) {
     constexpr int kB = 27 * N * 32;  // bytes of a chunk's weights
     constexpr int kB3 = kB / 3;      // of one dz of it
     extern __shared__ __align__(128) unsigned char smtc[];
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
     if (ok) done = mbar_wait(mbar + (nst - 1) % kZmA, ((nst - 1) / kZmA) & 1);
     if (__syncthreads_or(!done)) {
         done = false;
-        if (tid == 0) atomicExch(err, 1);
+        if (tid == 0) atomicExch(&g_tc_err, 1);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -400,10 +402,16 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(geo.cols));
 }
 
-int *tc_err_flag() {
-    static int *flag = nullptr;
-    if (!flag && cudaMalloc(&flag, sizeof(int)) == cudaSuccess) cudaMemset(flag, 0, sizeof(int));
-    return flag;
+// dynamic shared memory above 48 KB, asked for once per kernel and device
+// (`seen` holds the devices that granted it)
+template <typename K> bool allow_smem(K kern, int bytes, std::atomic<uint64_t> &seen) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (seen.load(std::memory_order_relaxed) & bit) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    seen.fetch_or(bit, std::memory_order_relaxed);
+    return true;
 }
 
 // the tcgen05 path: 16-byte aligned channel rows and weights (all three are
@@ -451,19 +459,13 @@ ZmGeo conv_geo(const Act &x) {
 template <int N>
 int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
     using Cfg = ZmCfg<N>;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv3_zm<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kMost) != cudaSuccess)
-            return BBMG_CUDA;
-        attr = true;
-    }
-    int *err = tc_err_flag();
-    if (!err) return BBMG_NO_MEMORY;
+    static std::atomic<uint64_t> seen{0};
+    if (!allow_smem(k_conv3_zm<N>, Cfg::kMost, seen)) return BBMG_CUDA;
     const ZmGeo g = conv_geo<N>(x);
     const long long grid = (long long)g.tw * g.th * x.n * g.tz;
     if (grid >= (1LL << 31)) return BBMG_BAD_ARGS;
     const int smem = Cfg::kFixed + (g.nb ? g.nb * Cfg::kB : kZmA * (Cfg::kB / 3));
-    k_conv3_zm<N><<<(unsigned)grid, 128, smem, s>>>(x, wt, bias, y, relu, g, err);
+    k_conv3_zm<N><<<(unsigned)grid, 128, smem, s>>>(x, wt, bias, y, relu, g);
     return done(cudaGetLastError());
 }
 
@@ -1024,12 +1026,8 @@ int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void
     // tensor cores: channel counts in whole tiles and 16-byte aligned channel rows
     if (!no_mma && ax.c % 16 == 0 && ag.c % 8 == 0 && ax.ld % 8 == 0 && ag.ld % 8 == 0 &&
         !(reinterpret_cast<uintptr_t>(ax.p) & 15) && !(reinterpret_cast<uintptr_t>(ag.p) & 15)) {
-        static bool attr = false;
-        if (!attr) {
-            if (cudaFuncSetAttribute(k_wgrad_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem) != cudaSuccess)
-                return BBMG_CUDA;
-            attr = true;
-        }
+        static std::atomic<uint64_t> seen{0};
+        if (!allow_smem(k_wgrad_mma, (int)kWgSmem, seen)) return BBMG_CUDA;
         const int tw = (ax.w + 15) / 16, th = (ax.h + 15) / 16, blocks = (ax.c / 16) * ((ag.c + 15) / 16);
         const long long cols = (long long)tw * th * ax.n;
         if (blocks > 65535 || cols * ax.d >= (1LL << 31)) return BBMG_BAD_ARGS;
@@ -1052,12 +1050,11 @@ int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void
 }
 
 int nn_tc_error(void) {
-    int *flag = tc_err_flag();
-    if (!flag) return BBMG_NO_MEMORY;
     int v = 0;
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpy(&v, flag, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    const int none = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpyFromSymbol(&v, g_tc_err, sizeof(int)) != cudaSuccess)
         return BBMG_CUDA;
-    if (v) cudaMemset(flag, 0, sizeof(int));
+    if (v && cudaMemcpyToSymbol(g_tc_err, &none, sizeof(int)) != cudaSuccess) return BBMG_CUDA;
     return v ? BBMG_CUDA : BBMG_OK;
 }
 

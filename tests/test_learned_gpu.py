@@ -9,6 +9,9 @@ accumulation error; FP32 outputs (weight gradients, head, loss) get 1e-4 of
 the magnitude of their terms.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -524,3 +527,11 @@ def test_convolution_of_a_packed_slice(L):
     dxg = torch.empty_like(xg)
     assert L.nn_conv3_dgrad(C.byref(act(yg, shape)), P(part), C.byref(act(dxg, shape)), None) == 0
     close_bf16(from_cl(dxg, shape), U.conv3_dgrad(from_cl(yg, shape), wt_))
+
+
+def test_first_convolution_under_capture():
+    """The first call of a process may be inside a stream capture: it allocates nothing."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.join(root, "tests", "conv_capture_probe.py")], cwd=root,
+                       env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "capture ok" in r.stdout, r.stdout + r.stderr
