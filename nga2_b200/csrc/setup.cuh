@@ -55,7 +55,7 @@ cudaError_t launch_restrict(const Lay &F, const Lay &C, const T *c2f, const T *r
 template <typename T>
 cudaError_t launch_prolong(const Lay &F, const Lay &C, const T *c2f, const T *vC, T *vF, cudaStream_t s);
 // vtail.cu: the coarsest solve; perm is the row permutation of the stored LU
-constexpr size_t kCoarseSmem = 200 * 1024;  // factors of up to 152 unknowns stay on chip
+constexpr size_t kCoarseSmem = 202 * 1024;  // factors of up to 160 unknowns stay on chip
 cudaError_t coarse_solve_prepare();  // per device, before the first coarse solve
 template <typename T>
 cudaError_t launch_coarse_solve(const Lay &L, const double *LU, const int *perm, const int *pinned, const T *f, T *v,

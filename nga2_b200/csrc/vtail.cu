@@ -37,17 +37,30 @@ namespace {
 // ---------------------------------------------------------------------------
 // coarsest level (bbmg_class.f90:891-927): the stored LU, FP64 always
 
-// x(i) of lane i % 32, register i / 32; A column major with ld rows, ld a
-// multiple of 8, the rows and columns beyond np those of a unit matrix.
+// The factors as the solve reads them, column major: staged in shared memory
+// with ld a multiple of 8, the rows and columns beyond np those of a unit
+// matrix, or as they lie in global memory, where reads beyond np give that.
+template <bool STAGED> struct Factors {
+    const double *A;
+    int np, ld;
+    __device__ __forceinline__ double at(int r, int c) const {
+        if (STAGED) return A[c * ld + r];
+        return r < np && c < np ? __ldg(A + c * np + r) : (r == c ? 1.0 : 0.0);
+    }
+};
+
+// x(i) of lane i % 32, register i / 32.
 // Eight unknowns at a time: every lane solves their small triangle itself (the
 // values come by eight independent shuffles), then updates its own rows with
 // them.  Each x(i) still loses its terms one by one in increasing (backward:
 // decreasing) order, so the values are those of the column-by-column solve;
 // the chain per unknown is a product and a difference instead of a shuffle,
-// a load and a store as well.
-template <int M>
-__device__ __forceinline__ void lu_solve_warp(const double *A, int ld, const int *__restrict__ pinned, int np,
-                                              int lane, double (&x)[M]) {
+// a load and a store as well.  From global memory a block of eight costs one L2
+// round trip (its coefficients do not depend on x) instead of eight.
+template <int M, bool STAGED>
+__device__ __forceinline__ void lu_solve_warp(const Factors<STAGED> &F, const int *__restrict__ pinned, int lane,
+                                              double (&x)[M]) {
+    const int np = F.np, rows = STAGED ? F.ld : np;
     unsigned pin[M];
 #pragma unroll
     for (int m = 0; m < M; m++) {
@@ -60,24 +73,22 @@ __device__ __forceinline__ void lu_solve_warp(const double *A, int ld, const int
         for (int l0 = 0; l0 < 32; l0 += 8) {
             const int k0 = 32 * mk + l0;
             if (k0 >= np) break;
-            const double *D = A + k0 * ld + k0;  // the block's triangle
             double xb[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) xb[j] = __shfl_sync(0xffffffffu, x[mk], l0 + j);
 #pragma unroll
             for (int j = 0; j < 7; j++)
 #pragma unroll
-                for (int i = j + 1; i < 8; i++) xb[i] = __dsub_rn(xb[i], __dmul_rn(xb[j], D[j * ld + i]));
+                for (int i = j + 1; i < 8; i++) xb[i] = __dsub_rn(xb[i], __dmul_rn(xb[j], F.at(k0 + i, k0 + j)));
 #pragma unroll
             for (int j = 0; j < 8; j++)
                 if (lane == l0 + j) x[mk] = xb[j];
 #pragma unroll
             for (int m = mk; m < M; m++) {
                 const int i = lane + 32 * m;
-                if (i >= k0 + 8 && i < ld) {
-                    const double *col = A + k0 * ld + i;
+                if (i >= k0 + 8 && i < rows) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) x[m] = __dsub_rn(x[m], __dmul_rn(xb[j], col[j * ld]));
+                    for (int j = 0; j < 8; j++) x[m] = __dsub_rn(x[m], __dmul_rn(xb[j], F.at(i, k0 + j)));
                 }
             }
         }
@@ -88,16 +99,15 @@ __device__ __forceinline__ void lu_solve_warp(const double *A, int ld, const int
         for (int l0 = 24; l0 >= 0; l0 -= 8) {
             const int k0 = 32 * mk + l0;
             if (k0 >= np) continue;
-            const double *D = A + k0 * ld + k0;
             double xb[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) xb[j] = __shfl_sync(0xffffffffu, x[mk], l0 + j);
 #pragma unroll
             for (int j = 7; j >= 0; j--) {
                 // a pinned unknown is zero whatever its pivot
-                xb[j] = (pin[mk] >> (l0 + j)) & 1u ? 0.0 : __ddiv_rn(xb[j], D[j * ld + j]);
+                xb[j] = (pin[mk] >> (l0 + j)) & 1u ? 0.0 : __ddiv_rn(xb[j], F.at(k0 + j, k0 + j));
 #pragma unroll
-                for (int i = 0; i < j; i++) xb[i] = __dsub_rn(xb[i], __dmul_rn(xb[j], D[j * ld + i]));
+                for (int i = 0; i < j; i++) xb[i] = __dsub_rn(xb[i], __dmul_rn(xb[j], F.at(k0 + i, k0 + j)));
             }
 #pragma unroll
             for (int j = 0; j < 8; j++)
@@ -106,9 +116,8 @@ __device__ __forceinline__ void lu_solve_warp(const double *A, int ld, const int
             for (int m = 0; m <= mk; m++) {
                 const int i = lane + 32 * m;
                 if (i < k0) {
-                    const double *col = A + k0 * ld + i;
 #pragma unroll
-                    for (int j = 7; j >= 0; j--) x[m] = __dsub_rn(x[m], __dmul_rn(xb[j], col[j * ld]));
+                    for (int j = 7; j >= 0; j--) x[m] = __dsub_rn(x[m], __dmul_rn(xb[j], F.at(i, k0 + j)));
                 }
             }
         }
@@ -152,26 +161,33 @@ __device__ __noinline__ void lu_solve_mem(const double *__restrict__ A, const in
     }
 }
 
-template <int M>
-__device__ __forceinline__ void lu_solve_regs(const double *A, const int *__restrict__ pinned, int np, int lane,
+template <int M, bool STAGED>
+__device__ __forceinline__ void lu_solve_regs(const Factors<STAGED> &F, const int *__restrict__ pinned, int lane,
                                               double *xs) {
     double x[M];
 #pragma unroll
-    for (int m = 0; m < M; m++) x[m] = lane + 32 * m < np ? xs[lane + 32 * m] : 0.0;
-    lu_solve_warp<M>(A, lu_ld(np), pinned, np, lane, x);
+    for (int m = 0; m < M; m++) x[m] = lane + 32 * m < F.np ? xs[lane + 32 * m] : 0.0;
+    lu_solve_warp<M, STAGED>(F, pinned, lane, x);
 #pragma unroll
     for (int m = 0; m < M; m++)
-        if (lane + 32 * m < np) xs[lane + 32 * m] = x[m];
+        if (lane + 32 * m < F.np) xs[lane + 32 * m] = x[m];
+}
+__device__ __noinline__ void lu_solve_l2(const double *__restrict__ LU, const int *__restrict__ pinned, int np,
+                                         int lane, double *xs) {
+    lu_solve_regs<5, false>(Factors<false>{LU, np, np}, pinned, lane, xs);
 }
 
 // xs: the row-permuted right-hand side in shared memory, replaced by the
-// solution; one warp.  Factors staged in shared memory at A (up to 152
-// unknowns), or LU in global memory.
+// solution; one warp.  Factors staged in shared memory at A (up to 131 unknowns
+// in the cluster, 160 in a launch of its own), or LU in global memory: eight
+// columns at a time while x fits five registers a lane, else column by column.
+// One cycle with 157 unknowns in the cluster: 203 us column by column, 136 us so.
 __device__ __forceinline__ void lu_solve(const double *A, const double *__restrict__ LU, bool staged,
                                          const int *__restrict__ pinned, int np, int lane, double *xs) {
-    if (!staged) lu_solve_mem(LU, pinned, np, lane, xs);
-    else if (np <= 64) lu_solve_regs<2>(A, pinned, np, lane, xs);
-    else lu_solve_regs<5>(A, pinned, np, lane, xs);
+    if (!staged && np > 160) lu_solve_mem(LU, pinned, np, lane, xs);
+    else if (!staged) lu_solve_l2(LU, pinned, np, lane, xs);
+    else if (np <= 64) lu_solve_regs<2, true>(Factors<true>{A, np, lu_ld(np)}, pinned, lane, xs);
+    else lu_solve_regs<5, true>(Factors<true>{A, np, lu_ld(np)}, pinned, lane, xs);
 }
 
 // The coarsest solve as a launch of its own (levels that are not fused): one

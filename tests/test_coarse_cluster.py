@@ -88,3 +88,25 @@ def test_cycle_leaves_the_vectors_of_every_level(monkeypatch, dims, per, prec):
     for n, (a, b) in enumerate(zip(*got)):
         for w in ("v", "f", "r"):
             assert np.array_equal(a[w], b[w]), (n + 1, w)
+
+
+@pytest.mark.parametrize("dims,unknowns", [((262, 2, 2), 131), ((22, 12, 4), 132), ((38, 8, 4), 152), ((34, 18, 2), 153),
+                                           ((20, 16, 4), 160), ((46, 14, 2), 161), ((12, 12, 12), 216)])
+def test_solves_around_the_sizes_of_the_coarsest_solve(dims, unknowns):
+    """In the cluster factors on chip up to 131 unknowns, read eight columns at a time up to 160, column by column
+    above; the solve as a launch of its own, on chip up to 160, at the same sizes."""
+    o, g = pair(dims, (True, False, False), seed=11, maxit=2, rcvg=0.0)
+    assert int(np.prod(g.level_dims(g.nlvl))) == unknowns
+    b = np.random.default_rng(12).standard_normal(dims[::-1])
+    b -= b.mean()
+    xo, _, ro = o.solve(b)
+    xg, _, rg, _ = g.solve(b)
+    assert ro == rg and np.array_equal(xo, xg)
+    n = g.nlvl
+    f = np.zeros(tuple(m + 2 for m in g.level_dims(n)[::-1]))
+    f[1:-1, 1:-1, 1:-1] = np.random.default_rng(13).standard_normal(tuple(g.level_dims(n)[::-1]))
+    o.put(n, "f", f)
+    g.put(n, "f", f)
+    o.direct_solve()
+    g.step("direct", n)
+    assert np.array_equal(g.get(n, "v"), o.get(n, "v"))
