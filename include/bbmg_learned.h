@@ -38,10 +38,11 @@ typedef struct {
 int nn_conv3(const nn_act *x, const void *wt, const float *bias, const nn_act *y, int relu, void *stream);
 
 /* How nn_conv3(x, wt, ..., y) or nn_conv3_dgrad(x, wt, y) would run: *tcgen05 = 1
- * on tcgen05.mma, 0 on mma.sync; on tcgen05 the output planes a tile holds and
- * its weight buffers (0: the weights come with each input plane).  Looks at the
- * sizes and addresses only and launches nothing. */
-int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers);
+ * on tcgen05.mma, 0 on mma.sync; on tcgen05 also the output planes a tile holds,
+ * its weight buffers (0: the weights come with each input plane) and the input
+ * planes in flight.  Looks at the sizes and addresses only and launches nothing. */
+int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers,
+                     int *slots);
 
 /* BBMG_CUDA if a tcgen05 convolution's completion wait ran out on the current
  * device since the last call (the flag is then cleared), else 0.  Synchronises

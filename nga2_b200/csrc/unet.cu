@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(128) k_conv3(Act x, const bf16 *__restrict__ w
 // ---------------------------------------------------------------------------
 // Convolution as implicit GEMM on the fifth-generation tensor cores (tcgen05).
 // A CTA owns a column of 8 (w) x 16 (h) voxels (M = 128) over up to DZ output
-// planes and all N = cout output channels; its FP32 accumulators, DZ x cout
-// columns, stay in TMEM.
+// planes and N output channels (all of them, or one of G groups: with_width); its FP32
+// accumulators, DZ x N columns, stay in TMEM.
 //   * K is walked in chunks of 16 input channels; a chunk marches over the
 //     DZ + 2 input planes.  A stage is one plane of one chunk: its 10 x 18
 //     voxels with the halo (periodic wrap), as [8-channel group][voxel][16 B],
@@ -136,25 +136,26 @@ __global__ void __launch_bounds__(128) k_conv3(Act x, const bf16 *__restrict__ w
 //   * Input plane p contributes to the output planes p-1, p, p+1 through the
 //     taps dz = +1, 0, -1.  Their accumulators are neighbouring TMEM columns and
 //     the chunk's weights are stored [dy, dx][group][dz][cout], so one MMA of
-//     N = 3 cout does all three: with 16 output channels an MMA's time is the
-//     reading of A (128 rows of 32 bytes at 128 B per cycle), whatever N.
-//     Where 3 cout > 256 the three go out one by one.
-//   * A planes sit in a ring of kZmA slots filled with cp.async kZmA - 1
-//     stages ahead; one thread issues a stage's MMAs and commits them to the
-//     slot's mbarrier, which gates its refill.  The weights of a chunk have NB
-//     buffers; with one, the next chunk's load waits for the MMAs before it.  A
-//     tile of one output plane has the weights of each stage's dz in its slot.
+//     up to 3 N columns does all three: with 16 output channels an MMA's time is
+//     the reading of A (128 rows of 32 bytes at 128 B per cycle), whatever N.
+//   * A planes sit in a ring of S slots filled with cp.async S - 1 stages ahead;
+//     one thread issues a stage's MMAs and commits them to the slot's mbarrier,
+//     which gates its refill.  The weights of a chunk have NB buffers; with one,
+//     the next chunk's load waits for the MMAs before it.  A tile of one output
+//     plane has the weights of each stage's dz in its slot.
 //   * The epilogue reads the four warps' 32 TMEM lanes, adds the bias, applies
 //     the ReLU and stores BF16.
 // Measured at 128^3 (the whole forward pass of the U-Net with its guess assembly):
 // 3.55 ms with one CTA per 128-voxel row tile that staged an input row for each
-// (dz, dy) and issued 27 MMAs of N = cout per tile, 1.71 ms with this kernel.
+// (dz, dy) and issued 27 MMAs of N = cout per tile, 1.32 ms with this kernel.  The
+// nine MMAs of a tile of one plane are unrolled: one thread issues them, and on
+// 8^3 64->64 takes 25 us with a loop and 20 without.
 // Every mbarrier wait is bounded: a wait that runs out raises g_tc_err (read by
 // nn_tc_error), and the CTA then drains its copies, frees its TMEM and returns
 // without writing.
 __device__ int g_tc_err;  // each device's own, there without an allocation: a first call may be captured
 constexpr unsigned kTcSpinLimit = 1u << 22;
-constexpr int kZmA = 4;                     // A slots
+constexpr int kZmA = 4;                     // A slots, or 2 (conv_geo)
 constexpr int kZmVox = 10 * 18;             // voxels of a halo plane
 constexpr int kZmPlane = kZmVox * 32;       // bytes of a stage's A
 
@@ -206,6 +207,7 @@ struct ZmGeo {
     int dz;          // output planes per tile
     int cols;        // TMEM columns
     int nb;          // weight buffers; 0: with one output plane per tile, weights in the plane's stage
+    int slots;       // A slots
 };
 
 __device__ __forceinline__ int wrapn(int i, int n) {
@@ -213,18 +215,23 @@ __device__ __forceinline__ int wrapn(int i, int n) {
     return i < 0 ? i + n : i;
 }
 
-template <int N>
+template <int N, int G, int S>
 __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict__ wt, const float *__restrict__ bias,
                                                    Act y, int relu, ZmGeo geo) {
+    static_assert(3 * N <= 256 && S >= 2 && S <= 4, "one MMA for three planes; the first S - 1 stages in one chunk");
     constexpr int kB = 27 * N * 32;  // bytes of a chunk's weights
     constexpr int kB3 = kB / 3;      // of one dz of it
     extern __shared__ __align__(128) unsigned char smtc[];
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(smtc);
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smtc + 16);  // kZmA barriers
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smtc + 16);  // S barriers
     unsigned char *A = smtc + 128;
-    unsigned char *B = A + (size_t)kZmA * kZmPlane;
+    unsigned char *B = A + (size_t)S * kZmPlane;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int cin = x.c, nchunk = cin >> 4;
+    constexpr int cout = G * N;
+    const int co0 = G == 1 ? 0 : blockIdx.y * N;  // this CTA's output channels
+    if (G > 1) wt += (long long)co0 * cin;
+    if (G > 1 && bias) bias += co0;
     int t = blockIdx.x;
     const int w0 = (t % geo.tw) * 8;
     t /= geo.tw;
@@ -240,7 +247,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0)
-        for (int s = 0; s < kZmA; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + s)));
+        for (int s = 0; s < S; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + s)));
 
     // this thread's copies of a plane: chunk e = tid + 128 u is group e & 1 of voxel e >> 1
     int src[3];
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
     auto load_a = [&](int st) {
         const int c = st / npl, r = st - c * npl;
         const bf16 *p = xn + (long long)wrapn(z0 - 1 + r, x.d) * zstride + c * 16;
-        unsigned char *As = A + (size_t)(st % kZmA) * kZmPlane;
+        unsigned char *As = A + (size_t)(st % S) * kZmPlane;
 #pragma unroll
         for (int u = 0; u < 3; u++) {
             const int e = tid + 128 * u;
@@ -267,7 +274,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         for (int e = tid; e < 54 * N; e += 128) {
             const int g = e & 1, o = (e >> 1) % N, tap = (e >> 1) / N;  // tap = 9 dz + 3 dy + dx
             const int dzi = tap / 9, t9 = tap - 9 * dzi;
-            cpa16(Bs + (((t9 * 2 + g) * 3 + 2 - dzi) * N + o) * 16, wt + ((long long)tap * N + o) * cin + c * 16 + g * 8);
+            cpa16(Bs + (((t9 * 2 + g) * 3 + 2 - dzi) * N + o) * 16, wt + ((long long)tap * cout + o) * cin + c * 16 + g * 8);
         }
     };
     // one output plane: stage st (input plane st % 3 of chunk st / 3) has only the
@@ -275,21 +282,20 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
     const bool third = geo.nb == 0;
     auto load_b3 = [&](int st) {
         const int c = st / 3, r = st - 3 * c;
-        unsigned char *Bs = B + (size_t)(st % kZmA) * kB3;
+        unsigned char *Bs = B + (size_t)(st % S) * kB3;
         for (int e = tid; e < 18 * N; e += 128) {
             const int g = e & 1, o = (e >> 1) % N, t9 = (e >> 1) / N;
-            cpa16(Bs + ((t9 * 2 + g) * N + o) * 16, wt + ((long long)(9 * r + t9) * N + o) * cin + c * 16 + g * 8);
+            cpa16(Bs + ((t9 * 2 + g) * N + o) * 16, wt + ((long long)(9 * r + t9) * cout + o) * cin + c * 16 + g * 8);
         }
     };
     auto commit_group = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
     if (!third) load_b(0);
 #pragma unroll 1
-    for (int p = 0; p < kZmA - 1; p++) {
+    for (int p = 0; p < S - 1; p++) {
         if (p < nst) {
             if (third) load_b3(p);
-            else if (p && p % npl == 0 && geo.nb > 1) load_b(p / npl);
-            load_a(p);
+            load_a(p);  // S - 1 <= npl: of the first chunk
         }
         commit_group();
     }
@@ -309,7 +315,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         const int c = st / npl, r = st - c * npl;
         if (st && r == 0 && geo.nb == 1) {
             // one weight buffer: the MMAs of the chunk before have to be done
-            const bool done = mbar_wait(mbar + (st - 1) % kZmA, ((st - 1) / kZmA) & 1);
+            const bool done = mbar_wait(mbar + (st - 1) % S, ((st - 1) / S) & 1);
             if (__syncthreads_or(!done)) {
                 ok = false;
                 break;
@@ -318,34 +324,33 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
             commit_group();
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kZmA - 2) : "memory");  // stage st has landed
+            asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");  // stage st has landed
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor core
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned as = smem_u32(A + (size_t)(st % kZmA) * kZmPlane), bs = smem_u32(third ? B + (size_t)(st % kZmA) * kB3 : B + (size_t)(c % geo.nb) * kB);
+            const unsigned as = smem_u32(A + (size_t)(st % S) * kZmPlane), bs = smem_u32(third ? B + (size_t)(st % S) * kB3 : B + (size_t)(c % geo.nb) * kB);
             // output planes lo .. hi (tile-local) of input plane r - 1
             const int lo = max(0, r - 2), hi = min(nq - 1, r), b0 = lo - (r - 2);
-            const int nblk = hi - lo + 1, per = 3 * N <= 256 ? nblk : 1;
-            const uint32_t idesc = umma_idesc_bf16(per * N);
+            const auto tap = [&](int t9) { return umma_desc(as + ((t9 / 3) * 10 + t9 % 3) * 16, kZmVox * 16, 160); };
+            if (third) {
+#pragma unroll
+                for (int t9 = 0; t9 < 9; t9++)
+                    umma_bf16(tmem, tap(t9), umma_desc(bs + t9 * 2 * N * 16, N * 16, 128), umma_idesc_bf16(N));
+            } else {
+                const uint32_t idesc = umma_idesc_bf16((hi - lo + 1) * N);
 #pragma unroll 1
-            for (int t9 = 0; t9 < 9; t9++) {
-                const uint64_t ad = umma_desc(as + ((t9 / 3) * 10 + t9 % 3) * 16, kZmVox * 16, 160);
-                if (third) {
-                    umma_bf16(tmem, ad, umma_desc(bs + t9 * 2 * N * 16, N * 16, 128), umma_idesc_bf16(N));
-                    continue;
-                }
-                for (int b = 0; b < nblk; b += per)
-                    umma_bf16(tmem + (lo + b) * N, ad, umma_desc(bs + (t9 * 6 + b0 + b) * N * 16, 3 * N * 16, 128), idesc);
+                for (int t9 = 0; t9 < 9; t9++)
+                    umma_bf16(tmem + lo * N, tap(t9), umma_desc(bs + (t9 * 6 + b0) * N * 16, 3 * N * 16, 128), idesc);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(smem_u32(mbar + st % kZmA)) : "memory");
+                         ::"r"(smem_u32(mbar + st % S)) : "memory");
         }
-        const int nx = st + kZmA - 1;  // the stage to fill next, in the slot stage st-1 used
+        const int nx = st + S - 1;  // the stage to fill next, in the slot stage st-1 used
         if (nx < nst) {
             if (st >= 1) {
-                const bool done = mbar_wait(mbar + nx % kZmA, ((st - 1) / kZmA) & 1);
+                const bool done = mbar_wait(mbar + nx % S, ((st - 1) / S) & 1);
                 if (__syncthreads_or(!done)) {
                     ok = false;
                     break;
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         commit_group();
     }
     bool done = false;
-    if (ok) done = mbar_wait(mbar + (nst - 1) % kZmA, ((nst - 1) / kZmA) & 1);
+    if (ok) done = mbar_wait(mbar + (nst - 1) % S, ((nst - 1) / S) & 1);
     if (__syncthreads_or(!done)) {
         done = false;
         if (tid == 0) atomicExch(&g_tc_err, 1);
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(128) k_conv3_zm(Act x, const bf16 *__restrict_
         const int h = h0 + (tid >> 3), w = w0 + (tid & 7);
         const bool in = h < x.h && w < x.w;
         for (int q = 0; q < nq; q++) {
-            bf16 *dst = y.p + ((((long long)n * x.d + z0 + q) * x.h + h) * x.w + w) * y.ld;
+            bf16 *dst = y.p + ((((long long)n * x.d + z0 + q) * x.h + h) * x.w + w) * y.ld + co0;
 #pragma unroll
             for (int c0 = 0; c0 < N; c0 += 16) {
                 unsigned v[16];
@@ -424,62 +429,70 @@ bool tc_eligible(const Act &x, const bf16 *wt, const Act &y) {
     return !(x.ld % 8 || y.ld % 8 || off16(x.p) || off16(wt) || off16(y.p));
 }
 
-template <int N> struct ZmCfg {
-    static constexpr int kFixed = 128 + kZmA * kZmPlane, kB = 27 * N * 32;
-    static constexpr int kTwoPerSm = 112 * 1024, kMost = 226 * 1024;
-    static_assert(kFixed + kB <= kMost, "one weight buffer has to fit");
-    static constexpr bool kThirds = kFixed + kZmA * (kB / 3) <= kMost;
-};
+// Wide outputs go in groups of 64 or 32 channels (with_width): with 96, 128 or 192
+// at once the weights of a tile of one plane fill an SM, whose copies then wait for
+// its MMAs.  At 128^3 64->128, 128->128, 32->96 and 64->192 take 3.84, 7.23, 1.79
+// and 5.77 ms so, 1.95, 3.67, 0.88 and 3.06 in groups; at 8^3, where more CTAs
+// cover more SMs, 35, 66, 17 and 52 us and 20, 37, 9 and 20.
+constexpr int zm_smem(int n, int slots, int nb) {
+    return 128 + slots * kZmPlane + (nb ? nb * 27 * n * 32 : slots * 9 * n * 32);
+}
+
+constexpr int kZmMost = 226 * 1024;
+static_assert(zm_smem(64, kZmA, 2) <= kZmMost, "the widest group has to fit");
 
 template <int N>
-ZmGeo conv_geo(const Act &x) {
-    using Cfg = ZmCfg<N>;
+ZmGeo conv_geo(const Act &x, int groups) {
+    constexpr int kTwoPerSm = 112 * 1024;
     ZmGeo g;
     g.tw = (x.w + 7) / 8;
     g.th = (x.h + 15) / 16;
     // output planes per tile: as many as 128 TMEM columns hold (four CTAs share
     // an SM's 512), fewer where that would leave SMs idle
-    const long long cols = (long long)g.tw * g.th * x.n;
-    g.dz = min(x.d, max(1, 128 / N));
+    const long long cols = (long long)g.tw * g.th * x.n * groups;
+    g.dz = min(x.d, 128 / N);
     while (g.dz > 1 && cols * ((x.d + g.dz - 1) / g.dz) < 2 * 148) g.dz = (g.dz + 1) / 2;
     g.tz = (x.d + g.dz - 1) / g.dz;
     for (g.cols = 32; g.cols < g.dz * N;) g.cols *= 2;
     // One plane per tile (the deep levels: few tiles, long K): each stage brings
     // the weights of its own dz, so that no load waits for a whole chunk's MMAs.
-    // Average per layer of the network's 64- and 128-channel convolutions on 64^3:
-    // 36 and 65 us with one weight buffer per chunk, 33 and 56 us so.
-    // Otherwise two weight buffers where two CTAs per SM still fit with them, or
-    // where only one fits anyway.
-    constexpr bool two = Cfg::kFixed + 2 * Cfg::kB <= Cfg::kTwoPerSm ||
-                         (Cfg::kFixed + Cfg::kB > Cfg::kTwoPerSm && Cfg::kFixed + 2 * Cfg::kB <= Cfg::kMost);
-    g.nb = g.dz == 1 && Cfg::kThirds ? 0 : (x.c > 16 && two ? 2 : 1);
+    // Otherwise two weight buffers where two CTAs per SM still fit with them.
+    g.nb = g.dz == 1 ? 0 : (x.c > 16 && zm_smem(N, kZmA, 2) <= kTwoPerSm ? 2 : 1);
+    // Two slots where that lets more CTAs share an SM and so ends in fewer waves.
+    // A wave of o2 CTAs per SM takes about (o2 + o4) / (2 o4) of the time of one
+    // of o4 (64->64: 45 us with 2, 56 with 3).  At 128^3 64->64 takes 1.24 ms with
+    // four slots and 1.04 with two; on 8x128x128 (1.7 against 1.2 waves, two of
+    // either) 95 and 99 us.
+    const long long ctas = cols * g.tz;
+    const auto per_sm = [&](int slots) { return min(512 / g.cols, 228 * 1024 / (zm_smem(N, slots, g.nb) + 1024)); };
+    const auto waves = [&](int o) { return (ctas + 148 * o - 1) / (148 * o); };
+    const int o2 = per_sm(2), o4 = per_sm(kZmA);
+    g.slots = o2 > o4 && waves(o2) * (o2 + o4) < waves(o4) * 2 * o4 ? 2 : kZmA;
     return g;
 }
 
-template <int N>
-int launch_conv_tc(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
-    using Cfg = ZmCfg<N>;
+template <int N, int G, int S>
+int launch_zm(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, const ZmGeo &g, cudaStream_t s) {
     static std::atomic<uint64_t> seen{0};
-    if (!allow_smem(k_conv3_zm<N>, Cfg::kMost, seen)) return BBMG_CUDA;
-    const ZmGeo g = conv_geo<N>(x);
+    if (!allow_smem(k_conv3_zm<N, G, S>, kZmMost, seen)) return BBMG_CUDA;
     const long long grid = (long long)g.tw * g.th * x.n * g.tz;
     if (grid >= (1LL << 31)) return BBMG_BAD_ARGS;
-    const int smem = Cfg::kFixed + (g.nb ? g.nb * Cfg::kB : kZmA * (Cfg::kB / 3));
-    k_conv3_zm<N><<<(unsigned)grid, 128, smem, s>>>(x, wt, bias, y, relu, g);
+    k_conv3_zm<N, G, S><<<dim3((unsigned)grid, G), 128, zm_smem(N, S, g.nb), s>>>(x, wt, bias, y, relu, g);
     return done(cudaGetLastError());
 }
 
-// f(output width as a constant) for the widths of tc_eligible
+// f(output channels of a CTA, groups) as constants, for the widths of tc_eligible
 template <typename F>
-int with_width(int n, F f) {
-    switch (n) {
-    case 16: return f(std::integral_constant<int, 16>{});
-    case 32: return f(std::integral_constant<int, 32>{});
-    case 48: return f(std::integral_constant<int, 48>{});
-    case 64: return f(std::integral_constant<int, 64>{});
-    case 96: return f(std::integral_constant<int, 96>{});
-    case 128: return f(std::integral_constant<int, 128>{});
-    case 192: return f(std::integral_constant<int, 192>{});
+int with_width(int cout, F f) {
+    using std::integral_constant;
+    switch (cout) {
+    case 16: return f(integral_constant<int, 16>{}, integral_constant<int, 1>{});
+    case 32: return f(integral_constant<int, 32>{}, integral_constant<int, 1>{});
+    case 48: return f(integral_constant<int, 48>{}, integral_constant<int, 1>{});
+    case 64: return f(integral_constant<int, 64>{}, integral_constant<int, 1>{});
+    case 96: return f(integral_constant<int, 32>{}, integral_constant<int, 3>{});
+    case 128: return f(integral_constant<int, 64>{}, integral_constant<int, 2>{});
+    case 192: return f(integral_constant<int, 64>{}, integral_constant<int, 3>{});
     }
     return BBMG_BAD_ARGS;
 }
@@ -487,7 +500,12 @@ int with_width(int n, F f) {
 int launch_conv(const Act &x, const bf16 *wt, const float *bias, const Act &y, int relu, cudaStream_t s) {
     const int blocks = (x.nvox + 63) / 64;
     if (tc_eligible(x, wt, y))
-        return with_width(y.c, [&](auto n) { return launch_conv_tc<decltype(n)::value>(x, wt, bias, y, relu, s); });
+        return with_width(y.c, [&](auto width, auto groups) {
+            constexpr int N = decltype(width)::value, G = decltype(groups)::value;
+            const ZmGeo g = conv_geo<N>(x, G);
+            return g.slots == 2 ? launch_zm<N, G, 2>(x, wt, bias, y, relu, g, s)
+                                : launch_zm<N, G, kZmA>(x, wt, bias, y, relu, g, s);
+        });
     // output widths of the U-Net: 16/32/64/128 forward; the data gradients
     // of the concatenated decoder inputs add 48/96/192
     if (y.c % 8) return BBMG_BAD_ARGS;
@@ -1003,16 +1021,18 @@ int nn_conv3_dgrad(const nn_act *dy, const void *wd, const nn_act *dx, void *str
     return launch_conv(act_of(dy), (const bf16 *)wd, nullptr, act_of(dx), 0, (cudaStream_t)stream);
 }
 
-int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers) {
-    if (bad_act(x) || bad_act(y) || !wt || !tcgen05 || !planes || !buffers) return BBMG_BAD_ARGS;
+int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcgen05, int *planes, int *buffers,
+                     int *slots) {
+    if (bad_act(x) || bad_act(y) || !wt || !tcgen05 || !planes || !buffers || !slots) return BBMG_BAD_ARGS;
     const Act ax = act_of(x), ay = act_of(y);
     *tcgen05 = tc_eligible(ax, (const bf16 *)wt, ay);
-    *planes = *buffers = 0;
+    *planes = *buffers = *slots = 0;
     if (!*tcgen05) return BBMG_OK;
-    return with_width(ay.c, [&](auto n) {
-        const ZmGeo g = conv_geo<decltype(n)::value>(ax);
+    return with_width(ay.c, [&](auto width, auto groups) {
+        const ZmGeo g = conv_geo<decltype(width)::value>(ax, decltype(groups)::value);
         *planes = g.dz;
         *buffers = g.nb;
+        *slots = g.slots;
         return BBMG_OK;
     });
 }

@@ -190,10 +190,9 @@ def test_unaligned_weights_do_not_take_the_16_byte_copies():
     def path(cin, cout, shape=(1, 5, 16, 8), xo=0, wo=0, yo=0, ld=0):
         x = NL.Act(0x10000000 + xo, *shape, cin, cin + ld)
         y = NL.Act(0x20000000 + yo, *shape, cout, cout)
-        tc, planes, buf = C.c_int(-1), C.c_int(-1), C.c_int(-1)
-        assert L.bbmg_debug_conv3(C.byref(x), 0x30000000 + wo, C.byref(y), C.byref(tc), C.byref(planes),
-                                  C.byref(buf)) == 0
-        return tc.value
+        r = [C.c_int(-1) for _ in range(4)]
+        assert L.bbmg_debug_conv3(C.byref(x), 0x30000000 + wo, C.byref(y), *map(C.byref, r)) == 0
+        return r[0].value
 
     for cin, cout in ((16, 16), (192, 64), (128, 128), (64, 192)):
         assert path(cin, cout) == 1

@@ -77,8 +77,8 @@ def packed(L, w):
 
 
 def tiling(L, x, wt, y):
-    """(tcgen05, output planes per tile, weight buffers) that a convolution would run with."""
-    r = [C.c_int(-1) for _ in range(3)]
+    """(tcgen05, output planes per tile, weight buffers, input planes in flight) that a convolution would run with."""
+    r = [C.c_int(-1) for _ in range(4)]
     assert L.bbmg_debug_conv3(C.byref(x), wt, C.byref(y), *map(C.byref, r)) == 0
     return tuple(v.value for v in r)
 
@@ -535,3 +535,29 @@ def test_first_convolution_under_capture():
     r = subprocess.run([sys.executable, os.path.join(root, "tests", "conv_capture_probe.py")], cwd=root,
                        env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "capture ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("cin,cout,shape,plan", [
+    # groups of 64 or 32 output channels; (output planes per tile, weight buffers, input planes in flight) of the
+    # tiling that the case is there for: one plane, several planes with a remainder, and many CTAs with two slots
+    (32, 96, (1, 5, 17, 9), (1, 0, 4)), (16, 192, (2, 3, 16, 24), (1, 0, 4)), (48, 128, (1, 7, 40, 40), (1, 0, 4)),
+    (16, 128, (1, 9, 60, 70), (2, 1, 2)), (32, 96, (1, 9, 72, 72), (4, 2, 2)), (32, 192, (1, 5, 64, 64), (1, 0, 2))])
+def test_wide_outputs_in_groups(L, cin, cout, shape, plan):
+    """Output widths that several CTAs share, against the oracle, forward and data gradient."""
+    rng = np.random.default_rng(3 * cin + cout)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    wt_ = bf(rng.standard_normal((27, cin, cout)) / np.sqrt(27 * cin))
+    b = torch.as_tensor(rng.standard_normal(cout) * 0.1, dtype=torch.float32)
+    xg = to_cl(x)
+    yg = torch.full((n * d * h * w, cout), float("nan"), dtype=torch.bfloat16, device="cuda")
+    wt, _ = packed(L, wt_.numpy())
+    bg = b.cuda()
+    assert tiling(L, act(xg, shape), P(wt), act(yg, shape)) == (1,) + plan
+    assert L.nn_conv3(C.byref(act(xg, shape)), P(wt), P(bg), C.byref(act(yg, shape)), 1, None) == 0
+    assert L.nn_tc_error() == 0
+    close_bf16(from_cl(yg, shape), torch.relu(U.conv3(x, wt_, b.double())))
+    # the same tiling as the gradient of a convolution from cout to cin channels
+    _, wd = packed(L, np.ascontiguousarray(wt_.numpy().transpose(0, 2, 1)))
+    assert L.nn_conv3_dgrad(C.byref(act(xg, shape)), P(wd), C.byref(act(yg, shape)), None) == 0
+    close_bf16(from_cl(yg, shape), U.conv3_dgrad(x, bf(wt_.numpy().transpose(0, 2, 1).copy())))
