@@ -999,6 +999,11 @@ int grid_elems(long long n) {
 
 // views the elementwise kernels take eight channels at a time
 bool vec8(const Act &a) { return a.c % 8 == 0 && a.ld % 8 == 0 && !(reinterpret_cast<uintptr_t>(a.p) & 15); }
+// Means and sums of eight children keep one channel per thread while the outputs
+// are few: there a thread's eight sums one after the other take longer than the
+// loads.  8192 outputs take 1.8 us with one channel per thread and 2.2 with eight,
+// 65536 2.05 and 2.3, 110592 2.37 and 2.31, 262144 3.5 and 2.4.
+bool small(const Act &a) { return (long long)a.nvox * a.c <= 148 * 640; }
 #define BB_CHANNELS(eight, view, kern, ...)                                                                          \
     do {                                                                                                             \
         if (eight)                                                                                                   \
@@ -1107,7 +1112,7 @@ static bool halves(const nn_act *big, const nn_act *small) {
 int nn_pool2(const nn_act *x, const nn_act *y, void *stream) {
     if (bad_act(x) || bad_act(y) || !halves(x, y)) return BBMG_BAD_ARGS;
     const Act a = act_of(x), b = act_of(y);
-    BB_CHANNELS(vec8(a) && vec8(b), b, k_pool2, a, b);
+    BB_CHANNELS(vec8(a) && vec8(b) && !small(b), b, k_pool2, a, b);
     return done(cudaGetLastError());
 }
 int nn_pool2_bwd(const nn_act *dy, const nn_act *dx, int accumulate, void *stream) {
@@ -1125,7 +1130,7 @@ int nn_up2(const nn_act *x, const nn_act *y, void *stream) {
 int nn_up2_bwd(const nn_act *dy, const nn_act *dx, void *stream) {
     if (bad_act(dy) || bad_act(dx) || !halves(dy, dx)) return BBMG_BAD_ARGS;
     const Act a = act_of(dy), b = act_of(dx);
-    BB_CHANNELS(vec8(a) && vec8(b), b, k_up2_bwd, a, b);
+    BB_CHANNELS(vec8(a) && vec8(b) && !small(b), b, k_up2_bwd, a, b);
     return done(cudaGetLastError());
 }
 

@@ -561,3 +561,17 @@ def test_wide_outputs_in_groups(L, cin, cout, shape, plan):
     _, wd = packed(L, np.ascontiguousarray(wt_.numpy().transpose(0, 2, 1)))
     assert L.nn_conv3_dgrad(C.byref(act(xg, shape)), P(wd), C.byref(act(yg, shape)), None) == 0
     close_bf16(from_cl(yg, shape), U.conv3_dgrad(x, bf(wt_.numpy().transpose(0, 2, 1).copy())))
+
+
+@pytest.mark.parametrize("shape,c", [((1, 6, 9, 10), 48), ((2, 4, 6, 8), 32), ((1, 12, 20, 28), 16), ((1, 12, 22, 28), 16)])
+def test_pooling_on_few_and_many_voxels(L, shape, c):
+    """Means and sums of children on both sides of the size from which a thread takes eight channels."""
+    n, d, h, w = shape
+    big = (n, 2 * d, 2 * h, 2 * w)
+    x = bf(np.random.default_rng(c + d).standard_normal((n, c) + big[1:]))
+    xg = to_cl(x)
+    y = torch.empty((n * d * h * w, c), dtype=torch.bfloat16, device="cuda")
+    assert L.nn_pool2(C.byref(act(xg, big)), C.byref(act(y, shape)), None) == 0
+    close_bf16(from_cl(y, shape), U.pool2(x))
+    assert L.nn_up2_bwd(C.byref(act(xg, big)), C.byref(act(y, shape)), None) == 0
+    close_bf16(from_cl(y, shape), U.pool2(x) * 8.0)
