@@ -223,6 +223,10 @@ int bbmg_debug_step(bbmg_handle *h, int step, int level, int arg, int prec);
  * BBMG_STEP_CYCLE times cycle(level) as the solve runs it, the single-launch
  * coarse levels included. */
 int bbmg_profile_step(bbmg_handle *h, int step, int level, int arg, int prec, int reps, double *ms);
+/* First level (from 1) of those that the solve runs inside one launch and the
+ * thread blocks of that launch, for precision prec (0 FP64, 1 FP32); 0 and 0 where
+ * every level runs pass by pass. */
+int bbmg_debug_cluster(bbmg_handle *h, int prec, int *level, int *blocks);
 /* dense coarsest matrix (row-major np x np), its LU (row-major, unit lower
  * below the diagonal) and pivots; any pointer may be NULL. */
 int bbmg_debug_direct(bbmg_handle *h, double *op, double *lu, int *piv, int *np);

@@ -59,6 +59,10 @@ int nn_conv3_dgrad(const nn_act *dy, const void *wd, const nn_act *dx, void *str
  * the channel rows are 16-byte aligned; on the CUDA cores otherwise. */
 int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void *stream);
 
+/* How nn_conv3_wgrad(x, dy, ...) would run: *tensor = 1 on the tensor cores, then
+ * the planes of the grid that a block sums up.  Launches nothing. */
+int bbmg_debug_conv3_wgrad(const nn_act *x, const nn_act *dy, int *tensor, int *planes);
+
 /* FP32 master weights [27][cin][cout] -> BF16 forward ([27][cout][cin]) and
  * backward ([27][cin][cout], taps mirrored) packings. */
 int nn_pack_weights(const float *w, int cin, int cout, void *wt, void *wd, void *stream);

@@ -33,7 +33,7 @@ STEP = {"relax": 0, "residual": 1, "restrict": 2, "prolong": 3, "cycle": 4, "dir
 EXPORTS = ["bbmg_default_params", "bbmg_create", "bbmg_setup", "bbmg_solve", "bbmg_set_convergence",
            "bbmg_set_residual_norm",
            "bbmg_set_stream", "bbmg_get_info", "bbmg_destroy", "bbmg_last_error", "bbmg_debug_get",
-           "bbmg_debug_put", "bbmg_debug_step", "bbmg_debug_direct", "bbmg_profile_step",
+           "bbmg_debug_put", "bbmg_debug_step", "bbmg_debug_direct", "bbmg_debug_cluster", "bbmg_profile_step",
            "bbmg_residual_norm_noalloc", "bbmg_set_precond_stage"]
 
 
@@ -97,6 +97,7 @@ def load(path: str = LIB_PATH):
     lib.bbmg_debug_put.restype = C.c_longlong
     lib.bbmg_debug_step.argtypes = [P, I, I, I, I]
     lib.bbmg_debug_direct.argtypes = [P, P, P, P, C.POINTER(C.c_int)]
+    lib.bbmg_debug_cluster.argtypes = [P, I, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.bbmg_profile_step.argtypes = [P, I, I, I, I, I, C.POINTER(C.c_double)]
     lib.bbmg_set_precond_stage.argtypes = [P, STAGE_FN, P, I, P, P]
     _LIB = lib
@@ -270,6 +271,12 @@ class BBMG:
         ms = C.c_double(0.0)
         self._check(self.lib.bbmg_profile_step(self.h, STEP[name], n, arg, prec, reps, C.byref(ms)))
         return ms.value
+
+    def cluster(self, prec=0):
+        """(first level, thread blocks) of the levels that a solve runs inside one launch; (0, 0): none."""
+        level, blocks = C.c_int(0), C.c_int(0)
+        self._check(self.lib.bbmg_debug_cluster(self.h, prec, C.byref(level), C.byref(blocks)))
+        return level.value, blocks.value
 
     def direct(self):
         npv = C.c_int(0)

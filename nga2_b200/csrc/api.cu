@@ -216,12 +216,14 @@ void choose_tail(bbmg_handle *h) {
     constexpr int pi = PrecIdx<T>::value;
     long long most = kTailCells;
     if (const char *env = getenv("BBMG_TAIL_CELLS")) most = atoll(env);
+    int widest = kTailClusterMax;
+    if (const char *env = getenv("BBMG_TAIL_BLOCKS")) widest = atoi(env) >= kTailClusterMax ? kTailClusterMax : 8;
     for (int n = 1; h->prm.ncycle == 1 && n < h->nlvl; n++) {
         const Lay &L = h->lv[n].L;
         if ((long long)L.nx * L.ny * L.nz > most) continue;
         TailArgs<T> A{};
         size_t smem = 0;
-        for (int blocks = kTailClusterMax; blocks >= 8; blocks /= 2) {
+        for (int blocks = widest; blocks >= 8; blocks /= 2) {
             if (!plan_tail<T>(h, n, blocks, &A, &smem) || !tail_fits<T>(blocks)) continue;
             h->tail_n0[pi] = n;
             h->tail_blocks[pi] = blocks;
@@ -1168,6 +1170,14 @@ int bbmg_profile_step(bbmg_handle *h, int step, int n, int arg, int prec, int re
     float t = 0.f;
     CU(h, cudaEventElapsedTime(&t, h->ev0, h->ev1));
     *ms = (double)t / reps;
+    return BBMG_OK;
+}
+
+int bbmg_debug_cluster(bbmg_handle *h, int prec, int *level, int *blocks) {
+    if (!h || prec < 0 || prec > 1 || !level || !blocks) return BBMG_BAD_ARGS;
+    const bool on = h->tail_n0[prec] && !h->tail_off;
+    *level = on ? h->tail_n0[prec] : 0;
+    *blocks = on ? h->tail_blocks[prec] : 0;
     return BBMG_OK;
 }
 

@@ -726,6 +726,23 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_mma(Act x, Act gy, float *
     }
 }
 
+// tensor cores: channel counts in whole tiles and 16-byte aligned channel rows
+bool wgrad_mma(const Act &x, const Act &gy) {
+    static const bool off = getenv("BBMG_NO_WGRAD_MMA") != nullptr;
+    return !off && x.c % 16 == 0 && gy.c % 8 == 0 && x.ld % 8 == 0 && gy.ld % 8 == 0 &&
+           !(reinterpret_cast<uintptr_t>(x.p) & 15) && !(reinterpret_cast<uintptr_t>(gy.p) & 15);
+}
+
+// planes per CTA: a CTA ends with 27 x 256 atomic additions, so as many planes
+// as leave two CTAs per SM
+int wgrad_planes(const Act &x, const Act &gy) {
+    const int blocks = (x.c / 16) * ((gy.c + 15) / 16);
+    const long long cols = (long long)((x.w + 15) / 16) * ((x.h + 15) / 16) * x.n;
+    int nz = x.d;
+    while (nz > 1 && cols * blocks * ((x.d + nz - 1) / nz) < 2 * 148) nz = (nz + 1) / 2;
+    return nz;
+}
+
 // ---------------------------------------------------------------------------
 __global__ void k_pack(const float *__restrict__ w, int cin, int cout, bf16 *__restrict__ wt, bf16 *__restrict__ wd) {
     const long long n = 27LL * cin * cout;
@@ -1050,25 +1067,26 @@ int bbmg_debug_conv3(const nn_act *x, const void *wt, const nn_act *y, int *tcge
     });
 }
 
+int bbmg_debug_conv3_wgrad(const nn_act *x, const nn_act *dy, int *tensor, int *planes) {
+    if (bad_act(x) || bad_act(dy) || !tensor || !planes) return BBMG_BAD_ARGS;
+    const Act ax = act_of(x), ag = act_of(dy);
+    *tensor = wgrad_mma(ax, ag);
+    *planes = *tensor ? wgrad_planes(ax, ag) : 0;
+    return BBMG_OK;
+}
+
 int nn_conv3_wgrad(const nn_act *x, const nn_act *dy, float *dw, float *db, void *stream) {
     if (bad_act(x) || bad_act(dy) || !dw || x->n != dy->n || x->d != dy->d || x->h != dy->h || x->w != dy->w ||
         dy->c > 256)
         return BBMG_BAD_ARGS;
     const Act ax = act_of(x), ag = act_of(dy);
-    static const bool no_mma = getenv("BBMG_NO_WGRAD_MMA") != nullptr;
-    // tensor cores: channel counts in whole tiles and 16-byte aligned channel rows
-    if (!no_mma && ax.c % 16 == 0 && ag.c % 8 == 0 && ax.ld % 8 == 0 && ag.ld % 8 == 0 &&
-        !(reinterpret_cast<uintptr_t>(ax.p) & 15) && !(reinterpret_cast<uintptr_t>(ag.p) & 15)) {
+    if (wgrad_mma(ax, ag)) {
         static std::atomic<uint64_t> seen{0};
         if (!allow_smem(k_wgrad_mma, (int)kWgSmem, seen)) return BBMG_CUDA;
         const int tw = (ax.w + 15) / 16, th = (ax.h + 15) / 16, blocks = (ax.c / 16) * ((ag.c + 15) / 16);
         const long long cols = (long long)tw * th * ax.n;
         if (blocks > 65535 || cols * ax.d >= (1LL << 31)) return BBMG_BAD_ARGS;
-        // planes per CTA: a CTA ends with 27 x 256 atomic additions, so as many
-        // planes as leave two CTAs per SM
-        int nz = ax.d;
-        while (nz > 1 && cols * blocks * ((ax.d + nz - 1) / nz) < 2 * 148) nz = (nz + 1) / 2;
-        const int tz = (ax.d + nz - 1) / nz;
+        const int nz = wgrad_planes(ax, ag), tz = (ax.d + nz - 1) / nz;
         k_wgrad_mma<<<dim3((unsigned)(cols * tz), blocks), kWgThreads, kWgSmem, (cudaStream_t)stream>>>(ax, ag, dw, db, tw, th, tz, nz);
         return done(cudaGetLastError());
     }

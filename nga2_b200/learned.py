@@ -59,6 +59,7 @@ def lib():
     sig = {
         "nn_conv3": [A, P, P, A, I, P],
         "bbmg_debug_conv3": [A, P, A] + [C.POINTER(I)] * 4,
+        "bbmg_debug_conv3_wgrad": [A, A, C.POINTER(I), C.POINTER(I)],
         "nn_conv3_dgrad": [A, P, A, P],
         "nn_conv3_wgrad": [A, A, P, P, P],
         "nn_pack_weights": [P, I, I, P, P, P],

@@ -33,6 +33,7 @@ def pair(dims, per, seed=3, **kw):
 @pytest.mark.parametrize("dims,per", SLABS)
 def test_slab_splits_bitexact(dims, per):
     o, g = pair(dims, per, maxit=3, rcvg=0.0)
+    assert g.cluster() == (1, 16)
     b = np.random.default_rng(5).standard_normal(dims[::-1])
     b -= b.mean()
     xo, ito, ro = o.solve(b)
@@ -96,6 +97,7 @@ def test_solves_around_the_sizes_of_the_coarsest_solve(dims, unknowns):
     """In the cluster factors on chip up to 131 unknowns, read eight columns at a time up to 160, column by column
     above; the solve as a launch of its own, on chip up to 160, at the same sizes."""
     o, g = pair(dims, (True, False, False), seed=11, maxit=2, rcvg=0.0)
+    assert g.cluster() == (1, 16)
     assert int(np.prod(g.level_dims(g.nlvl))) == unknowns
     b = np.random.default_rng(12).standard_normal(dims[::-1])
     b -= b.mean()
@@ -110,3 +112,73 @@ def test_solves_around_the_sizes_of_the_coarsest_solve(dims, unknowns):
     o.direct_solve()
     g.step("direct", n)
     assert np.array_equal(g.get(n, "v"), o.get(n, "v"))
+
+
+def solved(monkeypatch, dims, per, prec, env=(), seed=3, **kw):
+    """Solution, iterations and residual of a solve, and the cluster that it ran in, with BBMG_* settings."""
+    from nga2_b200.bbmg import BBMG, BBOX, FP64, MIXED
+    with monkeypatch.context() as m:
+        for k, v in dict(env).items():
+            m.setenv(k, v)
+        h = BBMG(*dims, *per, method=BBOX, precision=MIXED if prec else FP64, maxit=3, rcvg=0.0, **kw)
+    stc, opr = P.random_operator(*dims, per, seed=seed)
+    h.setup(stc, opr)
+    b = np.random.default_rng(5).standard_normal(dims[::-1])
+    b -= b.mean()
+    x, it, r, _ = h.solve(b)
+    cl = h.cluster(prec)
+    h.close()
+    return (x, it, r), cl
+
+
+def same(a, b):
+    return np.array_equal(a[0], b[0]) and a[1:] == b[1:]
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("dims,per", SLABS)
+def test_cluster_of_16_and_8_blocks_and_passes_give_the_same_bits(monkeypatch, dims, per, prec):
+    ref, off = solved(monkeypatch, dims, per, prec, {"BBMG_TAIL_CELLS": "0"})
+    assert off == (0, 0)
+    got, cl = solved(monkeypatch, dims, per, prec)
+    assert cl == (1, 16)
+    assert same(got, ref)
+    got, (level, blocks) = solved(monkeypatch, dims, per, prec, {"BBMG_TAIL_BLOCKS": "8"})
+    assert level >= 1 and blocks == 8  # slabs twice as high: not every first level fits
+    assert same(got, ref)
+
+
+@pytest.mark.parametrize("pre,post,direct", [(1, 2, True), (3, 1, True), (0, 3, True), (2, 2, False)])
+def test_single_precision_sweep_counts_and_relaxed_coarsest_level(monkeypatch, pre, post, direct):
+    kw = dict(relax_pre=pre, relax_post=post, use_direct_solve=direct)
+    dims, per = (20, 12, 18), (True, False, True)  # 5 cells in x on the third level
+    ref, _ = solved(monkeypatch, dims, per, 1, {"BBMG_TAIL_CELLS": "0"}, **kw)
+    got, cl = solved(monkeypatch, dims, per, 1, **kw)
+    assert cl == (1, 16) and same(got, ref)
+
+
+@pytest.mark.parametrize("cells", [None, "0"])
+@pytest.mark.parametrize("pre,post,direct", [(3, 3, True), (1, 2, True), (2, 2, False)])
+def test_odd_periodic_sizes_with_three_sweeps_bitexact(monkeypatch, cells, pre, post, direct):
+    """The all-even colour has cells that meet across an odd periodic wrap: it is run again after a backward
+    sweep, in the cluster and pass by pass."""
+    if cells:
+        monkeypatch.setenv("BBMG_TAIL_CELLS", cells)
+    o, g = pair((15, 12, 9), (True, False, True), maxit=2, rcvg=0.0, relax_pre=pre, relax_post=post,
+                use_direct_solve=direct)
+    assert g.cluster() == ((0, 0) if cells else (1, 16))
+    b = np.random.default_rng(6).standard_normal((9, 12, 15))
+    b -= b.mean()
+    xo, _, ro = o.solve(b)
+    xg, _, rg, _ = g.solve(b)
+    assert ro == rg and np.array_equal(xo, xg)
+
+
+@pytest.mark.parametrize("prec,level", [(0, 2), (1, 1)])
+def test_first_level_that_does_not_fit_beside_the_factors(monkeypatch, prec, level):
+    """33^3 in FP64 with 125 coarsest unknowns: the cluster starts a level below; in FP32 it holds the first."""
+    dims, per = (33, 33, 33), (True, True, True)
+    got, cl = solved(monkeypatch, dims, per, prec)
+    assert cl == (level, 16)
+    ref, _ = solved(monkeypatch, dims, per, prec, {"BBMG_TAIL_CELLS": "0"})
+    assert same(got, ref)

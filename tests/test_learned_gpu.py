@@ -420,9 +420,9 @@ def test_learned_guess_on_turbulence_sequence():
     (96, 32, 1, False, (1, 4, 4, 32)), (192, 64, 0, False, (2, 2, 4, 16)), (64, 128, 1, False, (1, 2, 2, 256)),
     (128, 128, 0, False, (1, 4, 4, 8)), (32, 96, 0, True, (1, 4, 4, 32)), (64, 192, 0, True, (1, 4, 8, 8))])
 def test_tcgen05_convolution(L, cin, cout, relu, dgrad, shape):
-    """Grids of whole 128-voxel tiles take the tcgen05 path (TMEM accumulator,
-    staged K ring): forward and data-gradient convolutions against the oracle,
-    and no completion timeout."""
+    """The tcgen05 path (TMEM accumulators, staged K ring) on small grids of whole and of
+    part tiles: forward and data-gradient convolutions against the oracle, and no
+    completion timeout."""
     rng = np.random.default_rng(100 + cin + cout)
     n, d, h, w = shape
     if dgrad:   # dy has cin channels, dx the forward's input channels (cout here)
@@ -467,8 +467,8 @@ def test_network_with_tcgen05_rows_matches_oracle():
 
 
 @pytest.mark.parametrize("cin,cout,shape", [
-    # one voxel per direction, sizes under and just over a tile of 8 x 16 voxels, odd sizes, two batches,
-    # plane counts around the tile's (16 planes at 16 channels, one at 192), one and several input chunks
+    # one voxel per direction, sizes under and just over a tile of 8 x 16 voxels, odd sizes, two batches, one and
+    # several input chunks; few voxels, so every tile has one output plane
     (16, 16, (1, 1, 1, 1)), (16, 16, (1, 17, 17, 9)), (32, 16, (2, 3, 15, 7)), (48, 64, (1, 5, 16, 8)),
     (16, 192, (1, 2, 18, 5)), (128, 128, (1, 3, 2, 2)), (96, 32, (1, 9, 5, 24))])
 def test_convolution_tile_edges(L, cin, cout, shape):
@@ -488,8 +488,8 @@ def test_convolution_tile_edges(L, cin, cout, shape):
 
 
 @pytest.mark.parametrize("cin,cout,shape", [
-    # one voxel, sizes under and just over a tile of 16 x 16 voxels, an odd plane count, two batches, a half
-    # block of output channels
+    # one voxel, sizes under and just over a tile of 16 x 16 voxels, two batches, a half block of output
+    # channels; few voxels, so every block sums one plane
     (16, 16, (1, 1, 1, 1)), (32, 48, (1, 5, 17, 18)), (48, 32, (2, 3, 16, 33)), (16, 24, (1, 2, 15, 16)),
     (128, 128, (1, 2, 2, 2))])
 def test_weight_gradient_tile_edges(L, cin, cout, shape):
@@ -575,3 +575,128 @@ def test_pooling_on_few_and_many_voxels(L, shape, c):
     close_bf16(from_cl(y, shape), U.pool2(x))
     assert L.nn_up2_bwd(C.byref(act(xg, big)), C.byref(act(y, shape)), None) == 0
     close_bf16(from_cl(y, shape), U.pool2(x) * 8.0)
+
+
+@pytest.mark.parametrize("cin,cout,shape,plan", [
+    # (output planes per tile, weight buffers, input planes in flight): several planes with a last tile of one, one
+    # and two weight buffers, one and several input chunks, four and two slots, ragged rows
+    (16, 16, (1, 33, 92, 96), (8, 1, 4)), (48, 16, (1, 37, 60, 61), (4, 2, 4)), (32, 32, (1, 19, 64, 63), (2, 2, 2)),
+    (32, 48, (1, 19, 62, 64), (2, 2, 4)), (32, 64, (1, 27, 64, 60), (2, 1, 4)), (64, 64, (1, 19, 64, 64), (2, 1, 2)),
+    (16, 32, (2, 19, 64, 64), (4, 1, 4))])
+def test_convolution_tiles_of_several_planes(L, cin, cout, shape, plan):
+    rng = np.random.default_rng(5 * cin + cout)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    wt_ = bf(rng.standard_normal((27, cin, cout)) / np.sqrt(27 * cin))
+    b = torch.as_tensor(rng.standard_normal(cout) * 0.1, dtype=torch.float32)
+    xg = to_cl(x)
+    yg = torch.full((n * d * h * w, cout), float("nan"), dtype=torch.bfloat16, device="cuda")
+    wt, _ = packed(L, wt_.numpy())
+    bg = b.cuda()
+    assert tiling(L, act(xg, shape), P(wt), act(yg, shape)) == (1,) + plan
+    assert L.nn_conv3(C.byref(act(xg, shape)), P(wt), P(bg), C.byref(act(yg, shape)), 0, None) == 0
+    assert L.nn_tc_error() == 0
+    close_bf16(from_cl(yg, shape), U.conv3(x, wt_, b.double()))
+
+
+def wgrad_plan(L, x, dy):
+    """(tensor cores, planes per block) that a weight gradient would run with."""
+    r = [C.c_int(-1) for _ in range(2)]
+    assert L.bbmg_debug_conv3_wgrad(C.byref(x), C.byref(dy), *map(C.byref, r)) == 0
+    return tuple(v.value for v in r)
+
+
+@pytest.mark.parametrize("cin,cout,shape,planes", [
+    # blocks that march over several planes, the last one over fewer; rows of whole and of ragged tiles
+    (48, 16, (1, 37, 64, 64), 5), (16, 16, (1, 25, 60, 90), 2), (16, 24, (2, 29, 64, 64), 4), (64, 64, (1, 10, 40, 48), 3)])
+def test_weight_gradient_over_several_planes(L, cin, cout, shape, planes):
+    rng = np.random.default_rng(11 * cin + cout)
+    n, d, h, w = shape
+    x = bf(rng.standard_normal((n, cin, d, h, w)))
+    dy = bf(rng.standard_normal((n, cout, d, h, w)))
+    dw = torch.zeros(27 * cin * cout, dtype=torch.float32, device="cuda")
+    db = torch.zeros(cout, dtype=torch.float32, device="cuda")
+    xg, dyg = to_cl(x), to_cl(dy)
+    assert wgrad_plan(L, act(xg, shape), act(dyg, shape)) == (1, planes)
+    assert L.nn_conv3_wgrad(C.byref(act(xg, shape)), C.byref(act(dyg, shape)), P(dw), P(db), None) == 0
+    rw, rb = U.conv3_wgrad(x, dy)
+    tol = 1e-4 * float(np.sqrt(n * d * h * w))  # FP32 sums of V unit products
+    np.testing.assert_allclose(dw.cpu().double().numpy().reshape(27, cin, cout), rw.numpy(), rtol=0, atol=tol)
+    np.testing.assert_allclose(db.cpu().double().numpy(), rb.numpy(), rtol=0, atol=tol)
+
+
+def test_views_without_16_byte_rows(L):
+    """Views whose pitch is even but no multiple of eight: convolutions on mma.sync, the weight gradient on the CUDA
+    cores, one channel per thread elsewhere with the bits of the eight-channel kernels."""
+    rng = np.random.default_rng(31)
+    sh, half, c, co = (1, 24, 16, 28), (1, 12, 8, 14), 32, 48
+
+    def pitched(t):  # the same rows two elements further apart
+        p = torch.zeros((t.shape[0], t.shape[1] + 2), dtype=t.dtype, device="cuda")
+        p[:, :t.shape[1]] = t
+        return p
+
+    def view(t, s, ch):
+        return act(t, s, ch)
+
+    x, y = (bf(rng.standard_normal((1, k) + sh[1:])) for k in (c, c))
+    s = bf(rng.standard_normal((1, c) + half[1:]))
+    xg, yg, sg = to_cl(x), to_cl(y), to_cl(s)
+    V = xg.shape[0]
+    # convolution, its data gradient, its weight gradient
+    wt_ = bf(rng.standard_normal((27, c, co)) / np.sqrt(27 * c))
+    wt, wd = packed(L, wt_.numpy())
+    xp, op = pitched(xg), torch.zeros((V, co + 2), dtype=torch.bfloat16, device="cuda")
+    assert tiling(L, view(xp, sh, c), P(wt), view(op, sh, co))[0] == 0
+    assert L.nn_conv3(C.byref(view(xp, sh, c)), P(wt), None, C.byref(view(op, sh, co)), 1, None) == 0
+    z = torch.zeros(co, dtype=torch.float64)
+    close_bf16(from_cl(op, sh, co), torch.relu(U.conv3(x, wt_, z)))
+    dxp = torch.zeros((V, c + 2), dtype=torch.bfloat16, device="cuda")
+    assert L.nn_conv3_dgrad(C.byref(view(op, sh, co)), P(wd), C.byref(view(dxp, sh, c)), None) == 0
+    close_bf16(from_cl(dxp, sh, c), U.conv3_dgrad(from_cl(op, sh, co), wt_))
+    dw, db = torch.zeros(27 * c * co, device="cuda"), torch.zeros(co, device="cuda")
+    assert wgrad_plan(L, view(xp, sh, c), view(op, sh, co)) == (0, 0)
+    assert L.nn_conv3_wgrad(C.byref(view(xp, sh, c)), C.byref(view(op, sh, co)), P(dw), P(db), None) == 0
+    rw, rb = U.conv3_wgrad(x, from_cl(op, sh, co))
+    tol = 1e-4 * float(np.sqrt(V))
+    np.testing.assert_allclose(dw.cpu().double().numpy().reshape(27, c, co), rw.numpy(), rtol=0, atol=tol)
+    np.testing.assert_allclose(db.cpu().double().numpy(), rb.numpy(), rtol=0, atol=tol)
+    assert float(op[:, co:].abs().max()) == 0.0 and float(dxp[:, c:].abs().max()) == 0.0
+
+    # elementwise: (call, outputs) on both kinds of view
+    def both(call, *tensors):
+        res = []
+        for f in (lambda t: t.clone(), pitched):
+            ts = [f(t) for t in tensors]
+            assert call(*ts) == 0
+            res.append([t[:, :k.shape[1]].clone() for t, k in zip(ts, tensors)])
+            assert all(float(t[:, k.shape[1]:].abs().sum()) == 0.0 for t, k in zip(ts, tensors))
+        assert all(torch.equal(a, b) for a, b in zip(*res))
+        return res[0]
+
+    A = C.byref
+    both(lambda a, b: L.nn_relu_bwd(A(view(a, sh, c)), A(view(b, sh, c)), None), xg, yg)
+    both(lambda a, b: L.nn_pool2(A(view(a, sh, c)), A(view(b, half, c)), None), xg, sg)
+    both(lambda a, b: L.nn_pool2_bwd(A(view(a, half, c)), A(view(b, sh, c)), 1, None), sg, xg)
+    both(lambda a, b: L.nn_up2(A(view(a, half, c)), A(view(b, sh, c)), None), sg, xg)
+    both(lambda a, b: L.nn_up2_bwd(A(view(a, sh, c)), A(view(b, half, c)), None), xg, sg)
+    f = torch.from_numpy(rng.standard_normal(V)).cuda()
+    fp, sc = (C.c_void_p * 1)(f.data_ptr()), (C.c_double * 1)(0.5)
+    both(lambda a: L.nn_embed(1, fp, sc, 1, A(view(a, sh, c)), None), xg)
+    w, hb = torch.randn(c, device="cuda"), torch.randn(1, device="cuda")
+    out = [torch.empty(V, device="cuda") for _ in range(2)]
+    it = iter(out)
+    both(lambda a: L.nn_head(A(view(a, sh, c)), P(w), P(hb), P(next(it)), None), xg)
+    assert torch.equal(*out)
+    g = torch.randn(V, device="cuda")
+    sums = [torch.zeros(c + 1, device="cuda") for _ in range(2)]
+    it = iter(sums)
+
+    def head_bwd(a, b):
+        t = next(it)
+        return L.nn_head_bwd(A(view(a, sh, c)), P(w), P(g), A(view(b, sh, c)), P(t), C.c_void_p(t.data_ptr() + 4 * c), None)
+
+    both(head_bwd, xg, yg)
+    ref = torch.cat([from_cl(xg, sh)[0].reshape(c, V) @ g.cpu().double(), g.cpu().double().sum()[None]])
+    for t in sums:  # FP32 sums of V unit products in any order
+        np.testing.assert_allclose(t.cpu().double().numpy(), ref.numpy(), rtol=0, atol=1e-4 * float(np.sqrt(V)))
