@@ -82,8 +82,10 @@ constexpr int kTailMax = 8;            // levels in one launch (kernel parameter
 constexpr int kTailThreads = 256;
 constexpr int kTailClusterMax = 16;    // blocks of the cluster (non-portable size; 8 if refused)
 // most cells of the first fused level: a 64^3 FP64 solve takes 4.19 ms with none
-// fused, 3.04 from 16^3 and 2.75 ms from 32^3; larger levels do not fit a cluster
-// of 16 blocks (65536 cells measured no different: the slab limit applies)
+// fused, 3.04 from 16^3 and 2.75 ms from 32^3.  64x32x32 still fits the slabs of 16
+// blocks, in FP32 (208 KB a block) though not in FP64 beside the staged factors of
+// 128 unknowns; fused there a 64x32x32 cycle takes 0.184 instead of 0.197 ms, but a
+// 256x128x128 mixed solve 12.86 instead of 12.39
 constexpr long long kTailCells = 36864;
 constexpr long long kTailBlockCells = 4096;  // most cells of a block's slab
 // levels this small run inside block 0: a pass over 8^3 cells takes 0.65e3 cycles

@@ -17,8 +17,10 @@
 // What bounds it: a pass is a chain of latencies (barrier 0.4e3 cycles, shared
 // memory loads, a sum in the reference's order, a division) of a few warps, no
 // longer a kernel launch or an L2 round trip for v; FP64 levels of 16^3 and 32^3
-// wait for their coefficients from L2.  With the levels below 8^3 fused and the
-// others one launch per colour, a 32^3 mixed solve took 3.13 ms and a 64^3 FP64
+// wait for their coefficients from L2, and with a 4- or 7-plane first level their
+// kernel spills (255 registers, 3.8 KB of stores and 1.3 KB of loads; 0.8 and 0.3
+// KB with 27 planes, FP32 none to speak of).  With the levels below 8^3 fused and
+// the others one launch per colour, a 32^3 mixed solve took 3.13 ms and a 64^3 FP64
 // one 4.19; fused from 32^3 they take 1.62 and 2.75 ms.  A cluster is scheduled
 // as a unit, so no block can wait on one that is not running, and no barrier
 // outlives its kernel.
